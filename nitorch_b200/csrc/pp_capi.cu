@@ -44,6 +44,23 @@ static const pp_launcher_t kLaunchers[4][3][ppk::K_NMODES] = {PP_TYPE(f32), PP_T
 #undef PP_TYPE
 #undef PP_ROW
 
+// Direct kernels compiled from direct_inst.cu, one launcher per (dtype, dim, mode).
+#define PD_DECL(S, D)                                                \
+  cudaError_t pp_direct_##S##_d##D##_m0(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_direct_##S##_d##D##_m1(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_direct_##S##_d##D##_m2(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_direct_##S##_d##D##_m3(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_direct_##S##_d##D##_m4(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_direct_##S##_d##D##_m5(int, const ppk::PPArgs&, cudaStream_t);
+PD_DECL(f32, 2) PD_DECL(f32, 3) PD_DECL(bf16, 2) PD_DECL(bf16, 3)
+#undef PD_DECL
+#define PD_ROW(S, D)                                                                          \
+  {pp_direct_##S##_d##D##_m0, pp_direct_##S##_d##D##_m1, pp_direct_##S##_d##D##_m2,          \
+   pp_direct_##S##_d##D##_m3, pp_direct_##S##_d##D##_m4, pp_direct_##S##_d##D##_m5}
+using pd_launcher_t = cudaError_t (*)(int ord, const ppk::PPArgs& a, cudaStream_t st);
+static const pd_launcher_t kDirect[2][2][6] = {{PD_ROW(f32, 2), PD_ROW(f32, 3)}, {PD_ROW(bf16, 2), PD_ROW(bf16, 3)}};
+#undef PD_ROW
+
 namespace ppk {
 thread_local char g_last_kernel[64] = "";
 void note_kernel(const char* family, int mode, int ord, int cb) {
@@ -108,9 +125,36 @@ void set_grid(const pp_tensor* t, int D, int64_t& sN, int64_t s[3], int64_t& sD)
 
 bool fits32(int64_t v) { return v < (int64_t(1) << 31) - 1; }
 
+// Whether the direct kernels (pp_direct.cuh) serve a call: 3-D linear and 2-D
+// linear to cubic stencils of float32 / bfloat16 images, plain or fused modes.
+// Higher orders, 64-bit offsets, deterministic scatters, coordinates computed
+// in the kernel and the interleaved accumulators keep their kernels.  Offsets
+// inside a batch item are 32-bit there (those of channels 64-bit, but for the
+// target's), so the element extent of every tensor must fit; batch items times
+// planes stay below 2^24 (the kernel divides them in float).
+bool direct_ok(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs& a) {
+  if (wide || (dtype != PP_FLOAT32 && dtype != PP_BFLOAT16) || mode > ppk::K_PUSHGRAD) return false;
+  if (!(D == 3 && ord == 1) && !(D == 2 && ord >= 1 && ord <= 3)) return false;
+  if (a.det_acc || (a.flags & (ppk::F_VEC | ppk::F_IDGRID | ppk::F_ADDSELF | ppk::F_AFFINE)) || !ppk::lanes_enabled())
+    return false;
+  int64_t grid = (D - 1) * a.grid_sD, gg = (D - 1) * a.gg_sD, trgt = (a.C - 1) * a.trgt_sC;
+  int64_t src = 0, out = (D - 1) * a.out_sK;
+  for (int d = 0; d < D; ++d) {
+    const int64_t t = a.trgt_size[d] - 1, s = a.src_size[d] - 1;
+    grid += t * a.grid_s[d];
+    gg += t * a.gg_s[d];
+    trgt += t * a.trgt_s[d];
+    src += s * a.src_s[d];
+    out += std::max(t, s) * a.out_s[d];
+  }
+  return fits32(grid) && fits32(gg) && fits32(trgt) && fits32(src) && fits32(out) && a.trgt_size[D - 2] <= 65535 &&
+         a.C > 0 && fits32(a.C) && a.N * (D == 3 ? a.trgt_size[0] : 1) < (1 << 24);
+}
+
 cudaError_t launch(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs& a, cudaStream_t st) {
   if (dtype < 0 || dtype > 3 || D < 1 || D > 3 || mode < 0 || mode >= ppk::K_NMODES) return cudaErrorInvalidValue;
   count_launch();
+  if (direct_ok(dtype, D, mode, ord, wide, a)) return kDirect[dtype == PP_FLOAT32 ? 0 : 1][D - 2][mode](ord, a, st);
   return kLaunchers[dtype][D - 1][mode](ord, wide, a, st);
 }
 

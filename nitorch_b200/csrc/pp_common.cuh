@@ -173,6 +173,34 @@ __device__ __forceinline__ void bspline_stencil(int p, T f, T (&w)[NT], T (&g)[N
   }
 }
 
+// The same weights and derivatives for one order of 1-3 known at compile time
+// and f in [0, 1]: the recurrence written out without its zero terms (which a
+// compiler must keep, 0 * x not being 0 for every float x), every term
+// non-negative as there.  Tap j's weight is M_p(f + p - j).
+template <int ORD, bool NEED_G>
+__device__ __forceinline__ void spline_weights(float f, float (&w)[ORD + 1], float (&g)[ORD + 1]) {
+  static_assert(ORD >= 1 && ORD <= 3, "orders 1-3");
+  const float e = 1.f - f;
+  if constexpr (ORD == 1) {
+    w[0] = e;
+    w[1] = f;
+    if (NEED_G) { g[0] = -1.f; g[1] = 1.f; }
+  } else {
+    const float b0 = 0.5f * f * f, b1 = fmaf(f, e, 0.5f), b2 = 0.5f * e * e;  // order 2: at f, f + 1, f + 2
+    if constexpr (ORD == 2) {
+      w[0] = b2; w[1] = b1; w[2] = b0;
+      if (NEED_G) { g[0] = -e; g[1] = e - f; g[2] = f; }
+    } else {
+      constexpr float t = 1.f / 3.f;
+      w[0] = e * b2 * t;
+      w[1] = fmaf(f + 2.f, b2, (1.f + e) * b1) * t;
+      w[2] = fmaf(f + 1.f, b1, (2.f + e) * b0) * t;
+      w[3] = f * b0 * t;
+      if (NEED_G) { g[0] = -b2; g[1] = b2 - b1; g[2] = b1 - b0; g[3] = b0; }
+    }
+  }
+}
+
 // Lowest support node.  Odd orders: floor(x) - (p-1)/2 (exact).  Even orders
 // subtract a half in double, like the reference (whose double literals
 // promote the float coordinate), so the node choice is bit-identical.

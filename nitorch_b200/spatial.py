@@ -160,7 +160,17 @@ def _brick_keys_fit(grid, src_size):
 _BRICK = (4, 4, 6)  # PP_BRICK_X, PP_BRICK_Y, PP_BRICK_Z
 
 
-def _order_for(grid, src_size):
+def _direct(grid, interpolation, dtype):
+    """The call runs the direct kernels (3-D linear, 2-D linear to cubic;
+    float32 / bfloat16 images), which take the points in the grid's own
+    order: no sort to pay for."""
+    dim = grid.dim() - 2
+    orders = {int(i) for i in interpolation[:dim]}
+    return (len(orders) == 1 and dtype in (torch.float32, torch.bfloat16) and grid.dtype == torch.float32
+            and not _deterministic and (dim == 3 and orders == {1} or dim == 2 and orders <= {1, 2, 3}))
+
+
+def _order_for(grid, src_size, interpolation, dtype):
     """(perm, brick_start, records) for the call, or Nones for the natural
     order.  3-D grids get the brick-major order (it also drives the brick
     kernels); 1-D / 2-D grids the source-sorted one."""
@@ -168,7 +178,7 @@ def _order_for(grid, src_size):
     if mode == "natural":
         return None, None, None
     nvox = grid.numel() // grid.shape[-1]
-    if mode == "auto" and nvox < _SORT_MIN_SAMPLES:
+    if mode == "auto" and (nvox < _SORT_MIN_SAMPLES or _direct(grid, interpolation, dtype)):
         return None, None, None
     if nvox >= (1 << 31):
         return None, None, None
@@ -268,9 +278,9 @@ def _grid32(grid):
     return grid
 
 
-def _opts(bound, interpolation, extrapolate, grid=None, src_size=None):
+def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, dtype=None):
     _check_opts(bound, interpolation)
-    perm, starts, recs = (_order_for(grid, src_size) if grid is not None and grid.is_cuda
+    perm, starts, recs = (_order_for(grid, src_size, interpolation, dtype) if grid is not None and grid.is_cuda
                           else (None, None, None))
     o = _lib.options([int(b) for b in bound], [int(i) for i in interpolation],
                      int(extrapolate), _lib.PP_DETERMINISTIC if _deterministic else 0,
@@ -323,7 +333,7 @@ def grid_pull(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], input.dtype)
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]),
                       dtype=input.dtype, device=input.device)
     with _On(input):
@@ -339,7 +349,7 @@ def grid_pull_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], input.dtype)
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     ws, nws = _workspace(gi) if gi is not None else (None, 0)
@@ -381,7 +391,7 @@ def grid_push(input, grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, input.shape[2:], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape)
+    opt = _opts(bound, interpolation, extrapolate, g, shape, input.dtype)
     out = torch.empty((grid.shape[0], input.shape[1], *shape), dtype=input.dtype, device=input.device)
     ws, nws = _workspace(out)
     with _On(input):
@@ -397,7 +407,7 @@ def grid_push_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], input.dtype)
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     with _On(input):
@@ -425,7 +435,7 @@ def grid_count(grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, grid.shape[1:-1], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape)
+    opt = _opts(bound, interpolation, extrapolate, g, shape, g.dtype)
     out = torch.empty((grid.shape[0], 1, *shape), dtype=g.dtype, device=grid.device)
     ws, nws = _workspace(out)
     with _On(grid):
@@ -440,7 +450,7 @@ def grid_count_backward(grad, grid, bound, interpolation, extrapolate):
     _require_cuda(grid)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], g.dtype)
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device)
     gr = grad.to(g.dtype)
     with _On(grid):
@@ -460,7 +470,7 @@ def grid_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], input.dtype)
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1], dim),
                       dtype=input.dtype, device=input.device)
@@ -480,7 +490,7 @@ def grid_pull_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:])
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], input.dtype)
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]), dtype=input.dtype,
                       device=input.device)
