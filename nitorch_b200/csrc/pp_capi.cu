@@ -61,6 +61,21 @@ using pd_launcher_t = cudaError_t (*)(int ord, const ppk::PPArgs& a, cudaStream_
 static const pd_launcher_t kDirect[2][2][6] = {{PD_ROW(f32, 2), PD_ROW(f32, 3)}, {PD_ROW(bf16, 2), PD_ROW(bf16, 3)}};
 #undef PD_ROW
 
+// Brick kernels compiled from brick_inst.cu, one launcher per (dtype, mode).
+#define PK_DECL(S)                                                \
+  cudaError_t pp_brick_##S##_m0(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_brick_##S##_m1(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_brick_##S##_m2(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_brick_##S##_m3(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_brick_##S##_m4(int, const ppk::PPArgs&, cudaStream_t); \
+  cudaError_t pp_brick_##S##_m5(int, const ppk::PPArgs&, cudaStream_t);
+PK_DECL(f32) PK_DECL(bf16)
+#undef PK_DECL
+#define PK_ROW(S) \
+  {pp_brick_##S##_m0, pp_brick_##S##_m1, pp_brick_##S##_m2, pp_brick_##S##_m3, pp_brick_##S##_m4, pp_brick_##S##_m5}
+static const pd_launcher_t kBrick[2][6] = {PK_ROW(f32), PK_ROW(bf16)};
+#undef PK_ROW
+
 namespace ppk {
 thread_local char g_last_kernel[64] = "";
 void note_kernel(const char* family, int mode, int ord, int cb) {
@@ -151,9 +166,25 @@ bool direct_ok(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs
          a.C > 0 && fits32(a.C) && a.N * (D == 3 ? a.trgt_size[0] : 1) < (1 << 24);
 }
 
+// Whether the brick kernels (pp_brick.cuh) serve a call: 3-D quadratic and
+// cubic stencils of float32 / bfloat16 images with at most four channels,
+// given a brick-major order.  The same exceptions as above; count's backward
+// pass (no target) keeps the per-point kernel.
+bool brick_ok(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs& a) {
+  if (wide || D != 3 || (dtype != PP_FLOAT32 && dtype != PP_BFLOAT16) || mode > ppk::K_PUSHGRAD) return false;
+  return (ord == 2 || ord == 3) && a.brick_start && a.perm && !a.det_acc && a.C >= 1 && a.C <= 4 &&
+         ppk::lanes_enabled() && !(a.flags & (ppk::F_AFFINE | ppk::F_IDGRID | ppk::F_ADDSELF | ppk::F_NOTRGT)) &&
+         fits32(a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2]);
+}
+
 cudaError_t launch(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs& a, cudaStream_t st) {
   if (dtype < 0 || dtype > 3 || D < 1 || D > 3 || mode < 0 || mode >= ppk::K_NMODES) return cudaErrorInvalidValue;
   count_launch();
+  if (brick_ok(dtype, D, mode, ord, wide, a)) {
+    // the pull's backward pass with both gradients is two kernels
+    if (mode == ppk::K_PUSHGRAD && (a.flags & ppk::F_A) && (a.flags & ppk::F_GRAD)) count_launch();
+    return kBrick[dtype == PP_FLOAT32 ? 0 : 1][mode](ord, a, st);
+  }
   if (direct_ok(dtype, D, mode, ord, wide, a)) return kDirect[dtype == PP_FLOAT32 ? 0 : 1][D - 2][mode](ord, a, st);
   return kLaunchers[dtype][D - 1][mode](ord, wide, a, st);
 }

