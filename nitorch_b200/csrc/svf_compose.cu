@@ -20,10 +20,32 @@
 
 namespace {
 
+// Points of both kernels: a CTA is a tile of 8 x 32 voxels (y, z), a thread
+// its (y, z) on `run` consecutive planes, so that a voxel's coordinates cost
+// no division.  Planes are numbered n * X + x over the batch.
+constexpr int SVF_TZ = 32, SVF_TY = 8, SVF_THREADS = SVF_TZ * SVF_TY;
+
+struct PlaneRun {
+  int o, end, n, x;  // plane, end of the run, batch item, x
+  __device__ __forceinline__ PlaneRun(int block, int run, int outer, int X) {
+    o = block * run;
+    end = min(o + run, outer);
+    n = o / X;
+    x = o - n * X;
+  }
+  __device__ __forceinline__ bool step(int X) {  // whether the next plane starts a batch item
+    ++o;
+    if (++x < X) return false;
+    x = 0;
+    ++n;
+    return true;
+  }
+};
+
 struct ComposeArgs {
   int32_t size[3], bound[3];
-  int32_t extrapolate, pad;
-  int64_t nvox;
+  int32_t extrapolate, outer, run;
+  float lo, hi[3];     // field of view: [lo, hi)
   int64_t fN, oN;      // batch strides
   int32_t fs[3], fC;   // field strides (elements): spatial, component
   int32_t os[3], oC;   // output strides
@@ -45,31 +67,31 @@ __device__ __forceinline__ void load3(const float* p, int fC, float (&v)[3]) {
 }
 
 template <bool UV4, bool OV4>
-__global__ void __launch_bounds__(256, UV4 ? 4 : 5) svf_compose_lin3(const ComposeArgs A) {
-  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < A.nvox; i += step) {
-    int sub[3];
-    int64_t n;
-    {
-      int64_t r = i;
-      sub[2] = static_cast<int>(r % A.size[2]); r /= A.size[2];
-      sub[1] = static_cast<int>(r % A.size[1]); r /= A.size[1];
-      sub[0] = static_cast<int>(r % A.size[0]);
-      n = r / A.size[0];
-    }
-    const float* un = A.u + n * A.fN;
-    const int base = sub[0] * A.fs[0] + sub[1] * A.fs[1] + sub[2] * A.fs[2];
-    float self[3], x[3];
-    load3<UV4>(un + base, A.fC, self);
+__global__ void __launch_bounds__(SVF_THREADS, UV4 ? 4 : 5) svf_compose_lin3(const __grid_constant__ ComposeArgs A) {
+  const int z = static_cast<int>(blockIdx.x) * SVF_TZ + (static_cast<int>(threadIdx.x) & 31);
+  const int y = static_cast<int>(blockIdx.y) * SVF_TY + (static_cast<int>(threadIdx.x) >> 5);
+  if (z >= A.size[2] || y >= A.size[1]) return;
+  PlaneRun P(static_cast<int>(blockIdx.z), A.run, A.outer, A.size[0]);
+  auto at_u = [&](const PlaneRun& q) { return A.u + q.n * A.fN + (q.x * A.fs[0] + y * A.fs[1] + z * A.fs[2]); };
+  float next[3];  // the next plane's voxel, read one ahead
+  load3<UV4>(at_u(P), A.fC, next);
+  while (P.o < P.end) {
+    const int sub[3] = {P.x, y, z};
+    const float* un = A.u + P.n * A.fN;
+    float* o = A.out + P.n * A.oN + (P.x * A.os[0] + y * A.os[1] + z * A.os[2]);
+    const float self[3] = {next[0], next[1], next[2]};
+    float x[3];
+    P.step(A.size[0]);
+    if (P.o < P.end) load3<UV4>(at_u(P), A.fC, next);
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[d] = static_cast<float>(sub[d]) + self[d];
-    float* o = A.out + n * A.oN + sub[0] * A.os[0] + sub[1] * A.os[1] + sub[2] * A.os[2];
-    const float tol = (A.extrapolate & 2) ? 0.55f : 0.05f;
     bool inb = true;
+    if (!(A.extrapolate & 1)) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) inb = inb && ppk::in_fov<float>(x[d], A.size[d], tol);
+      for (int d = 0; d < 3; ++d) inb = inb && x[d] >= A.lo && x[d] < A.hi[d];
+    }
     float res[3];
-    if (!((A.extrapolate & 1) || inb)) {  // outside the field of view: the identity term alone
+    if (!inb) {  // outside the field of view: the identity term alone
 #pragma unroll
       for (int d = 0; d < 3; ++d) res[d] = self[d];
     } else {
@@ -83,18 +105,24 @@ __global__ void __launch_bounds__(256, UV4 ? 4 : 5) svf_compose_lin3(const Compo
         const int i0 = static_cast<int>(f);
         const float t = xc - f;
         const int nn = A.size[d];
+        const int bd = A.bound[d];
+        w[d][0] = 1.f - t;
+        w[d][1] = t;
         if (i0 >= 0 && i0 + 1 < nn) {
           off[d][0] = i0 * A.fs[d];
           off[d][1] = off[d][0] + A.fs[d];
-          w[d][0] = 1.f - t;
-          w[d][1] = t;
+        } else if (bd != ppk::BND_DST1 && bd != ppk::BND_DST2 && bd != ppk::BND_ZERO) {
+          // bounds that map every node to one of the volume (signs cost the
+          // edge warps as much again)
+          off[d][0] = ppk::bound_index<int>(bd, i0, nn) * A.fs[d];
+          off[d][1] = ppk::bound_index<int>(bd, i0 + 1, nn) * A.fs[d];
         } else {
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            const int s = ppk::bound_sign<int>(A.bound[d], i0 + k, nn);
-            const int idx = s ? ppk::bound_index<int>(A.bound[d], i0 + k, nn) : 0;
+            const int s = ppk::bound_sign<int>(bd, i0 + k, nn);
+            const int idx = s ? ppk::bound_index<int>(bd, i0 + k, nn) : 0;
             off[d][k] = idx * A.fs[d];
-            w[d][k] = static_cast<float>(s) * (k ? t : 1.f - t);
+            w[d][k] *= static_cast<float>(s);
           }
         }
       }
@@ -130,146 +158,263 @@ __global__ void __launch_bounds__(256, UV4 ? 4 : 5) svf_compose_lin3(const Compo
 // Its adjoint with respect to u, for g = d loss / d out: the push of g
 // through the cell's eight corners, the grid gradient sum_c g_c grad(u_c),
 // and the identity term g, into a four-slot channel-interleaved float
-// accumulator (acc[v * 4 + c]) with one vector reduction per corner.  A
-// thread per voxel, consecutive lanes consecutive voxels along the last
-// axis: for a smooth field a voxel's upper-z corner is often the next
-// lane's lower-z corner, so the two contributions are added in registers
-// (one shuffle) and one reduction is saved.  Both lanes test the same
-// equality on valid addresses, so every contribution is added once.
+// accumulator (acc[v * 4 + c]) by vector reductions (red.global.add.v4.f32).
+// Nine reductions of 16 bytes per voxel, unmerged, bind on their sectors
+// through L2, so corners that neighbours share are summed in registers first:
+//   * along x, a thread keeps the four upper-x corners of its cell; at the
+//     next plane, a smooth field's cell is the one above, and they join its
+//     four lower-x corners.  Otherwise they are reduced as they are;
+//   * along z, a lane's upper-z corners are the next lane's lower-z corners
+//     when that lane's cell is the next along z: handed over by shuffles;
+//   * the voxel's own term (g and the grid gradient) joins the corner of its
+//     cell that is the voxel itself, when there is one.
+// A smooth field then takes about two reductions per voxel.  Cells are
+// compared by their unbounded node indices: equal nodes have equal addresses
+// under every bound.  Cells past the volume's edge stay on the merged path
+// under bounds without signs: with a path of their own, run for a lane or two
+// in every warp at the edge, they took a third of the kernel.
+// 160 x 192 x 160: 0.169 -> 0.113 ms per composition (the kernel before merged
+// along z only and took its coordinates from 64-bit divisions), forward 0.080
+// -> 0.064 ms.  Bound by issue (65 % active, ~515 instructions per voxel and
+// warp); the reductions are at 44 % of L2.
 struct ComposeBwdArgs {
   int32_t size[3], bound[3];
-  int32_t extrapolate, pad;
-  int64_t nvox;
+  int32_t extrapolate, outer, run;
+  float lo, hi[3];
   int64_t fN, gN, aN;
   int32_t fs[3], fC;   // field strides
   int32_t gs[3], gC;   // gradient strides
-  int32_t as[3], pad2; // accumulator strides (floats): Y*Z*4, Z*4, 4
+  int32_t as[3];       // accumulator strides (floats): Y*Z*4, Z*4, 4
   const float* u;
   const float* g;
   float* acc;
 };
 
-template <bool UV4>
-__global__ void __launch_bounds__(256, 5) svf_compose_backward_lin3(const ComposeBwdArgs A) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const bool live = i < A.nvox;
-  int sub[3] = {0, 0, 0};
-  int64_t n = 0;
-  if (live) {
-    int64_t r = i;
-    sub[2] = static_cast<int>(r % A.size[2]); r /= A.size[2];
-    sub[1] = static_cast<int>(r % A.size[1]); r /= A.size[1];
-    sub[0] = static_cast<int>(r % A.size[0]);
-    n = r / A.size[0];
-  }
-  const float* un = A.u + n * A.fN;
-  float gv[3] = {0.f, 0.f, 0.f}, x[3] = {0.f, 0.f, 0.f};
-  bool active = false;
-  if (live) {
-    const int fb = sub[0] * A.fs[0] + sub[1] * A.fs[1] + sub[2] * A.fs[2];
-    const float* gp = A.g + n * A.gN + sub[0] * A.gs[0] + sub[1] * A.gs[1] + sub[2] * A.gs[2];
-    float uu[3];
-    load3<UV4>(un + fb, A.fC, uu);
+__device__ __forceinline__ void red3(float* p, const float (&v)[3]) {
+  const float q[4] = {v[0], v[1], v[2], 0.f};
+  ppk::red_vec<4>(p, q);
+}
+
+template <bool UV4, bool GV4>
+__global__ void __launch_bounds__(SVF_THREADS, 3) svf_compose_backward_lin3(const __grid_constant__ ComposeBwdArgs A) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int z = static_cast<int>(blockIdx.x) * SVF_TZ + lane;
+  const int y = static_cast<int>(blockIdx.y) * SVF_TY + (static_cast<int>(threadIdx.x) >> 5);
+  const bool in_tile = z < A.size[2] && y < A.size[1];
+  // the upper-x corners of the last cell: values, accumulator offset of the
+  // first and steps to the others, and the cell they are the lower-x corners of
+  float up[2][2][3];
+  int up_at = 0, up_dy = 0, up_dz = 0, up_cell[3] = {0, 0, 0};
+  bool pending = false;
+  PlaneRun P(static_cast<int>(blockIdx.z), A.run, A.outer, A.size[0]);
+  float* acc = A.acc + P.n * A.aN;
+  auto flush = [&]() {
+    float* p = acc + up_at;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) red3(p + ((j ? up_dy : 0) + (k ? up_dz : 0)), up[j][k]);
+    pending = false;
+  };
+  float nu[3] = {0.f, 0.f, 0.f}, ng[3] = {0.f, 0.f, 0.f};  // the next plane's field and gradient, read one ahead
+  auto fetch = [&]() {
+    if (!in_tile) return;
+    load3<UV4>(A.u + P.n * A.fN + (P.x * A.fs[0] + y * A.fs[1] + z * A.fs[2]), A.fC, nu);
+    load3<GV4>(A.g + P.n * A.gN + (P.x * A.gs[0] + y * A.gs[1] + z * A.gs[2]), A.gC, ng);
+  };
+  fetch();
+  while (P.o < P.end) {
+    const float* un = A.u + P.n * A.fN;
+    const int px = P.x;
+    const float gv[3] = {ng[0], ng[1], ng[2]};
+    const float x[3] = {static_cast<float>(px) + nu[0], static_cast<float>(y) + nu[1], static_cast<float>(z) + nu[2]};
+    const bool last = P.step(A.size[0]);
+    if (P.o < P.end) fetch();
+    bool active = in_tile;
+    if (!(A.extrapolate & 1)) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) active = active && x[d] >= A.lo && x[d] < A.hi[d];
+    }
+    // the cell and the offset in it
+    int cell[3];
+    float t[3];
+    int idx[3], dn[3];  // lower node's index, steps to the upper node
+    bool inside = active;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      x[d] = static_cast<float>(sub[d]) + uu[d];
-      gv[d] = __ldg(gp + d * A.gC);
-    }
-    const float tol = (A.extrapolate & 2) ? 0.55f : 0.05f;
-    bool inb = true;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) inb = inb && ppk::in_fov<float>(x[d], A.size[d], tol);
-    active = (A.extrapolate & 1) || inb;
-  }
-  float* acc_n = A.acc + n * A.aN;
-  // per axis: the two nodes (field offsets, accumulator offsets, -1: none),
-  // weights and derivative weights with the boundary sign folded in
-  int fo[3][2], ao[3][2];
-  float w[3][2], dw[3][2];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float xc = fminf(fmaxf(x[d], -1073741824.f), 1073741824.f);
-    const float f = floorf(xc);
-    const int i0 = static_cast<int>(f);
-    const float t = xc - f;
-    const int nn = A.size[d];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      int s = 1, idx = i0 + k;
-      if (!(i0 >= 0 && i0 + 1 < nn)) {
-        s = ppk::bound_sign<int>(A.bound[d], i0 + k, nn);
-        idx = s ? ppk::bound_index<int>(A.bound[d], i0 + k, nn) : 0;
-      }
-      const bool ok = active && s != 0;
-      fo[d][k] = idx * A.fs[d];
-      ao[d][k] = ok ? idx * A.as[d] : -1;
-      w[d][k] = ok ? static_cast<float>(s) * (k ? t : 1.f - t) : 0.f;
-      dw[d][k] = ok ? static_cast<float>(s) * (k ? 1.f : -1.f) : 0.f;
-    }
-  }
-  // grid gradient: og_d = sum over corners of (derivative along d of the
-  // corner weight) * <g, u(corner)>
-  float og0 = 0.f, og1 = 0.f, og2 = 0.f;
-  if (active) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float sx = 0.f, dx = 0.f;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (ao[0][q] < 0 || ao[1][j] < 0 || ao[2][k] < 0) continue;  // a node outside: no tap
-          float cu[3];
-          load3<UV4>(un + fo[0][q] + fo[1][j] + fo[2][k], A.fC, cu);
-          const float dot = gv[0] * cu[0] + gv[1] * cu[1] + gv[2] * cu[2];
-          sx = fmaf(w[0][q], dot, sx);
-          dx = fmaf(dw[0][q], dot, dx);
+      const float xc = fminf(fmaxf(x[d], -1073741824.f), 1073741824.f);
+      const float f = floorf(xc);
+      cell[d] = static_cast<int>(f);
+      t[d] = xc - f;
+      idx[d] = cell[d];
+      dn[d] = 1;
+      if (cell[d] < 0 || cell[d] + 1 >= A.size[d]) {
+        // past the edge: bounds that map every node to one of the volume
+        // stay on this path
+        const int bd = A.bound[d];
+        if (bd == ppk::BND_DST1 || bd == ppk::BND_DST2 || bd == ppk::BND_ZERO) {
+          inside = false;
+        } else {
+          idx[d] = ppk::bound_index<int>(bd, cell[d], A.size[d]);
+          dn[d] = ppk::bound_index<int>(bd, cell[d] + 1, A.size[d]) - idx[d];
         }
-        og0 = fmaf(w[1][j] * w[2][k], dx, og0);
-        og1 = fmaf(dw[1][j] * w[2][k], sx, og1);
-        og2 = fmaf(w[1][j] * dw[2][k], sx, og2);
       }
     }
-  }
-  // the push of g, corner pairs (k = 0, 1) merged with the neighbouring lanes
+    float self[3] = {gv[0], gv[1], gv[2]};  // the voxel's own term
+    const float w[3][2] = {{1.f - t[0], t[0]}, {1.f - t[1], t[1]}, {1.f - t[2], t[2]}};
+    bool own = false;  // ... joins a corner of its cell
+    const int sx = px - cell[0], sy = y - cell[1], sz = z - cell[2];
+    if (inside) {
+      // grid gradient: og_d = sum over corners of (derivative along d of the
+      // corner weight) * <g, u(corner)>
+      const float* uc = un + (idx[0] * A.fs[0] + idx[1] * A.fs[1] + idx[2] * A.fs[2]);
+      const int fx = dn[0] * A.fs[0], fy = dn[1] * A.fs[1], fz = dn[2] * A.fs[2];
+      float yv[2], yx[2], yy[2];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
+      for (int k = 0; k < 2; ++k) {
+        float sv[2], sd[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float c0[3], c1[3];
+          const float* p = uc + ((j ? fy : 0) + (k ? fz : 0));
+          load3<UV4>(p, A.fC, c0);
+          load3<UV4>(p + fx, A.fC, c1);
+          const float d0 = fmaf(gv[2], c0[2], fmaf(gv[1], c0[1], gv[0] * c0[0]));
+          const float d1 = fmaf(gv[2], c1[2], fmaf(gv[1], c1[1], gv[0] * c1[0]));
+          sv[j] = fmaf(w[0][1], d1, w[0][0] * d0);
+          sd[j] = d1 - d0;
+        }
+        yv[k] = fmaf(w[1][1], sv[1], w[1][0] * sv[0]);
+        yx[k] = fmaf(w[1][1], sd[1], w[1][0] * sd[0]);
+        yy[k] = sv[1] - sv[0];
+      }
+      self[0] += fmaf(w[2][1], yx[1], w[2][0] * yx[0]);
+      self[1] += fmaf(w[2][1], yy[1], w[2][0] * yy[0]);
+      self[2] += yv[1] - yv[0];
+      own = ((sx | sy | sz) & ~1) == 0;
+    } else if (active) {
+      // bounds with signs or missing nodes: per node, every corner by itself
+      int fo[3][2], ao[3][2];
+      float ws[3][2], dw[3][2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int nn = A.size[d];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int s = ppk::bound_sign<int>(A.bound[d], cell[d] + k, nn);
+          const int idx = s ? ppk::bound_index<int>(A.bound[d], cell[d] + k, nn) : 0;
+          fo[d][k] = idx * A.fs[d];
+          ao[d][k] = s ? idx * A.as[d] : -1;
+          ws[d][k] = static_cast<float>(s) * w[d][k];
+          dw[d][k] = static_cast<float>(s) * (k ? 1.f : -1.f);
+        }
+      }
+      float og[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        const int fz = k ? fo[2][1] : fo[2][0], az = k ? ao[2][1] : ao[2][0];
+        const float wz = k ? ws[2][1] : ws[2][0], dz = k ? dw[2][1] : dw[2][0];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float sx_ = 0.f, dx_ = 0.f;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if ((ao[0][q] | ao[1][j] | az) < 0) continue;  // a corner without a node: no tap
+            float cu[3];
+            load3<UV4>(un + fo[0][q] + fo[1][j] + fz, A.fC, cu);
+            const float dot = gv[0] * cu[0] + gv[1] * cu[1] + gv[2] * cu[2];
+            sx_ = fmaf(ws[0][q], dot, sx_);
+            dx_ = fmaf(dw[0][q], dot, dx_);
+            const float wt = ws[0][q] * ws[1][j] * wz;
+            const float v[3] = {wt * gv[0], wt * gv[1], wt * gv[2]};
+            red3(acc + (ao[0][q] + ao[1][j] + az), v);
+          }
+          og[0] = fmaf(ws[1][j] * wz, dx_, og[0]);
+          og[1] = fmaf(dw[1][j] * wz, sx_, og[1]);
+          og[2] = fmaf(ws[1][j] * dz, sx_, og[2]);
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) self[d] += og[d];
+    }
+    if (in_tile && !own) red3(acc + (px * A.as[0] + y * A.as[1] + z * A.as[2]), self);
+
+    const bool joins = pending && inside && up_cell[0] == cell[0] && up_cell[1] == cell[1] && up_cell[2] == cell[2];
+    if (pending && !joins) flush();
+    // upper-z corners go to the next lane when they are its lower-z corners
+    const int cx = __shfl_down_sync(0xffffffffu, cell[0], 1), cy = __shfl_down_sync(0xffffffffu, cell[1], 1),
+              cz = __shfl_down_sync(0xffffffffu, cell[2], 1);
+    const unsigned ins = __ballot_sync(0xffffffffu, inside);
+    const bool gives = lane < 31 && inside && ((ins >> lane) & 2u) && cx == cell[0] && cy == cell[1] && cz == cell[2] + 1;
+    const unsigned given = __ballot_sync(0xffffffffu, gives);
+    const bool takes = lane > 0 && ((given >> (lane - 1)) & 1u);
+    const int at = idx[0] * A.as[0] + idx[1] * A.as[1] + idx[2] * 4, dy = dn[1] * A.as[1], dz = dn[2] * 4;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const bool xy = ao[0][q] >= 0 && ao[1][j] >= 0;
-      const int a0 = xy && ao[2][0] >= 0 ? ao[0][q] + ao[1][j] + ao[2][0] : -1;
-      const int a1 = xy && ao[2][1] >= 0 ? ao[0][q] + ao[1][j] + ao[2][1] : -1;
-      const float wxy = w[0][q] * w[1][j];
-      float v0[4] = {wxy * w[2][0] * gv[0], wxy * w[2][0] * gv[1], wxy * w[2][0] * gv[2], 0.f};
-      const float c1 = wxy * w[2][1];
-      // batch items differ: the neighbour's address is compared within one item
-      const int64_t nn_prev = __shfl_up_sync(0xffffffffu, n, 1);
-      const int64_t nn_next = __shfl_down_sync(0xffffffffu, n, 1);
-      const int prev_a1 = __shfl_up_sync(0xffffffffu, a1, 1);
-      const int next_a0 = __shfl_down_sync(0xffffffffu, a0, 1);
-      const float p0 = __shfl_up_sync(0xffffffffu, c1 * gv[0], 1);
-      const float p1 = __shfl_up_sync(0xffffffffu, c1 * gv[1], 1);
-      const float p2 = __shfl_up_sync(0xffffffffu, c1 * gv[2], 1);
-      const bool take_prev = lane > 0 && a0 >= 0 && prev_a1 == a0 && nn_prev == n;
-      const bool given_next = lane < 31 && a1 >= 0 && next_a0 == a1 && nn_next == n;
-      if (take_prev) {
-        v0[0] += p0;
-        v0[1] += p1;
-        v0[2] += p2;
+      // lower-x corners: this cell's, the pending ones, the own term
+      float lo[2][3];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float wyz = w[1][j] * w[2][k], w0 = w[0][0] * wyz, w1 = w[0][1] * wyz;
+        const bool me = own && sy == j && sz == k, me0 = me && sx == 0, me1 = me && sx == 1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          lo[k][c] = w0 * gv[c];
+          if (joins) lo[k][c] += up[j][k][c];
+          if (me0) lo[k][c] += self[c];
+          up[j][k][c] = w1 * gv[c];
+          if (me1) up[j][k][c] += self[c];
+        }
       }
-      if (a0 >= 0) ppk::red_vec<4>(acc_n + a0, v0);
-      if (a1 >= 0 && !given_next) {
-        const float v1[4] = {c1 * gv[0], c1 * gv[1], c1 * gv[2], 0.f};
-        ppk::red_vec<4>(acc_n + a1, v1);
+      if (given) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float v = __shfl_up_sync(0xffffffffu, lo[1][c], 1);
+          if (takes) lo[0][c] += v;
+        }
       }
+      float* p = acc + (at + (j ? dy : 0));
+      if (inside) red3(p, lo[0]);
+      if (inside && !gives) red3(p + dz, lo[1]);
+    }
+    pending = inside;
+    up_cell[0] = cell[0] + 1;
+    up_cell[1] = cell[1];
+    up_cell[2] = cell[2];
+    up_at = at + dn[0] * A.as[0];
+    up_dy = dy;
+    up_dz = dz;
+    if (last) {  // the next plane is another batch item's: its own accumulator
+      if (pending) flush();
+      acc = A.acc + P.n * A.aN;
     }
   }
-  // the identity term and the grid gradient at the voxel itself
-  if (live) {
-    const float vs[4] = {gv[0] + og0, gv[1] + og1, gv[2] + og2, 0.f};
-    ppk::red_vec<4>(acc_n + sub[0] * A.as[0] + sub[1] * A.as[1] + sub[2] * A.as[2], vs);
+  if (pending) flush();
+}
+
+template <class Args> void set_fov(Args& A) {
+  const float tol = (A.extrapolate & 2) ? 0.55f : 0.05f;
+  A.lo = -tol;
+  for (int d = 0; d < 3; ++d) A.hi[d] = static_cast<float>(A.size[d] - 1) + tol;
+}
+
+// Planes per thread, up to `most`: the number whose CTAs fill the resident
+// ones' waves best (long runs share more, and pay the start of a run less
+// often: `start` planes' worth); 0 where the grid does not fit a launch.
+int plane_run(const int32_t (&size)[3], int64_t outer, int resident, int most, double start, dim3& grid) {
+  const int64_t gz = (size[2] + SVF_TZ - 1) / SVF_TZ, gy = (size[1] + SVF_TY - 1) / SVF_TY;
+  const int64_t slots = int64_t(148) * resident;
+  int64_t run = 1;
+  double best = 0.;
+  for (int64_t r = 1; r <= most && r <= outer; ++r) {
+    const int64_t ctas = gz * gy * ((outer + r - 1) / r), waves = (ctas + slots - 1) / slots;
+    const double cost = static_cast<double>(waves) * (r + start);
+    if (r == 1 || cost < best) { best = cost; run = r; }
   }
+  if ((outer + run - 1) / run > 65535) run = (outer + 65534) / 65535;
+  if (gy > 65535 || outer >= (int64_t(1) << 31) - run) return 0;
+  grid = dim3(static_cast<unsigned>(gz), static_cast<unsigned>(gy), static_cast<unsigned>((outer + run - 1) / run));
+  return static_cast<int>(run);
 }
 
 bool fits_int(int64_t v) { return v < (int64_t(1) << 31) - 1; }
@@ -310,19 +455,21 @@ int svf_compose_linear3(const pp_tensor* disp, const pp_tensor* out, const int32
   A.fN = disp->strides[0];
   A.oN = out->strides[0];
   A.extrapolate = extrapolate;
-  A.pad = 0;
-  A.nvox = disp->sizes[0] * disp->sizes[1] * disp->sizes[2] * disp->sizes[3];
+  set_fov(A);
   A.u = static_cast<const float*>(disp->data);
   A.out = static_cast<float*>(out->data);
-  if (A.nvox == 0) return PP_OK;
-  const int64_t want = (A.nvox + 255) / 256;
-  const unsigned nb = static_cast<unsigned>(want < 148 * 32 ? want : 148 * 32);
+  if (numel(disp) == 0) return PP_OK;
+  dim3 nb;
+  const int64_t outer = disp->sizes[0] * disp->sizes[1];
+  A.run = plane_run(A.size, outer, 4, 8, 0.5, nb);
+  if (!A.run) return PP_ERR_UNSUPPORTED;
+  A.outer = static_cast<int32_t>(outer);
   ppk::note_kernel("svf_compose_lin3", ppk::K_PULL, 1, 3);
   const bool uv4 = padded4(disp), ov4 = padded4(out);
-  if (uv4 && ov4) svf_compose_lin3<true, true><<<nb, 256, 0, st>>>(A);
-  else if (uv4) svf_compose_lin3<true, false><<<nb, 256, 0, st>>>(A);
-  else if (ov4) svf_compose_lin3<false, true><<<nb, 256, 0, st>>>(A);
-  else svf_compose_lin3<false, false><<<nb, 256, 0, st>>>(A);
+  if (uv4 && ov4) svf_compose_lin3<true, true><<<nb, SVF_THREADS, 0, st>>>(A);
+  else if (uv4) svf_compose_lin3<true, false><<<nb, SVF_THREADS, 0, st>>>(A);
+  else if (ov4) svf_compose_lin3<false, true><<<nb, SVF_THREADS, 0, st>>>(A);
+  else svf_compose_lin3<false, false><<<nb, SVF_THREADS, 0, st>>>(A);
   count_launch();
   return cuda_check(cudaGetLastError(), "svf compose launch");
 }
@@ -354,19 +501,22 @@ int svf_compose_backward_linear3(const pp_tensor* grad, const pp_tensor* disp, f
   A.gN = grad->strides[0];
   A.aN = V * 4;
   A.extrapolate = extrapolate;
-  A.pad = A.pad2 = 0;
-  A.nvox = disp->sizes[0] * V;
+  set_fov(A);
   A.u = static_cast<const float*>(disp->data);
   A.g = static_cast<const float*>(grad->data);
   A.acc = acc;
-  if (A.nvox == 0) return PP_OK;
-  const int64_t nb = (A.nvox + 255) / 256;  // a thread per voxel: whole warps of consecutive voxels
-  if (nb > 0x7fffffffLL) return PP_ERR_UNSUPPORTED;
+  if (numel(disp) == 0) return PP_OK;
+  dim3 nb;
+  const int64_t outer = disp->sizes[0] * disp->sizes[1];
+  A.run = plane_run(A.size, outer, 3, 32, 1.0, nb);
+  if (!A.run) return PP_ERR_UNSUPPORTED;
+  A.outer = static_cast<int32_t>(outer);
   ppk::note_kernel("svf_compose_backward_lin3", ppk::K_PUSHGRAD, 1, 3);
-  if (padded4(disp))
-    svf_compose_backward_lin3<true><<<static_cast<unsigned>(nb), 256, 0, st>>>(A);
-  else
-    svf_compose_backward_lin3<false><<<static_cast<unsigned>(nb), 256, 0, st>>>(A);
+  const bool uv4 = padded4(disp), gv4 = padded4(grad);
+  if (uv4 && gv4) svf_compose_backward_lin3<true, true><<<nb, SVF_THREADS, 0, st>>>(A);
+  else if (uv4) svf_compose_backward_lin3<true, false><<<nb, SVF_THREADS, 0, st>>>(A);
+  else if (gv4) svf_compose_backward_lin3<false, true><<<nb, SVF_THREADS, 0, st>>>(A);
+  else svf_compose_backward_lin3<false, false><<<nb, SVF_THREADS, 0, st>>>(A);
   count_launch();
   return cuda_check(cudaGetLastError(), "svf compose backward launch");
 }
