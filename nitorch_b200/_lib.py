@@ -230,4 +230,23 @@ def options(bound, order, extrapolate, flags=0, sample_order=None, brick_start=N
 
 
 def stream_of(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(t.device.index))
+
+
+class On:
+    """Make `t`'s device current for the duration of a launch."""
+    __slots__ = ("dev", "prev")
+
+    def __init__(self, t):
+        self.dev = t.device.index
+        self.prev = None
+
+    def __enter__(self):
+        cur = torch._C._cuda_getDevice()  # (a CUDA tensor exists: the runtime is up)
+        if self.dev is not None and cur != self.dev:
+            self.prev = cur
+            torch.cuda.set_device(self.dev)
+
+    def __exit__(self, *exc):
+        if self.prev is not None:
+            torch.cuda.set_device(self.prev)

@@ -36,6 +36,12 @@ class _Layout:
         return out.reshape(*self.lead, *self.chan, *out.shape[2:])
 
 
+def _broadcast(a, b):
+    """torch.broadcast_shapes, which takes as long as a small call's launch,
+    only where the shapes differ."""
+    return a if a == b else torch.broadcast_shapes(a, b)
+
+
 def _fold(grid, image=None, shared_space=False):
     """Fold ``grid`` (*g_lead, *g_space, D) and ``image``
     (*i_lead, [C], *i_space) into kernel layout.  An image with exactly D
@@ -52,8 +58,8 @@ def _fold(grid, image=None, shared_space=False):
     i_lead = image.shape[:-dim - 1] if has_chan else ()
     i_space = image.shape[-dim:]
     if shared_space:
-        g_space = i_space = torch.broadcast_shapes(g_space, i_space)
-    lead = torch.broadcast_shapes(g_lead, i_lead)
+        g_space = i_space = _broadcast(g_space, i_space)
+    lead = _broadcast(g_lead, torch.Size(i_lead))
     folded_grid = grid.expand(*lead, *g_space, dim).reshape(-1, *g_space, dim)
     folded_image = image.expand(*lead, nchan or 1, *i_space).reshape(-1, nchan or 1, *i_space)
     chan = (nchan,) if nchan else ((1,) if len(lead) else ())
@@ -241,18 +247,18 @@ def resize(image, factor=None, shape=None, affine=None, anchor="c", dim=None, *a
     prefilter = kwargs.pop("prefilter", True)
     batch = image.shape[:-nb_dim]
     x = image.reshape(-1, 1, *inshape)
-    gdt = torch.float64 if x.dtype == torch.float64 else torch.float32
-    mat = torch.zeros((nb_dim, nb_dim + 1), dtype=gdt, device=x.device)
-    for d in range(nb_dim):
-        mat[d, d] = scales[d]
-        mat[d, nb_dim] = shifts[d]
     if prefilter:
         x = spline_coeff_nd(x, interpolation=interpolation, bound=bound, dim=nb_dim)
     if nb_dim == 3 and all(s > 0 for s in scales) and resize_supported(x, interpolation):
         # diagonal map: the separable kernel (equal to the affine pull)
         out = resize_pull(x, scales, shifts, outshape, interpolation, bound, extrapolate)
     else:
-        out = affine_pull(x, mat, outshape, interpolation, bound, extrapolate)
+        gdt = torch.float64 if x.dtype == torch.float64 else torch.float32
+        mat = torch.zeros((nb_dim, nb_dim + 1), dtype=gdt)
+        for d in range(nb_dim):
+            mat[d, d] = scales[d]
+            mat[d, nb_dim] = shifts[d]
+        out = affine_pull(x, mat.to(x.device), outshape, interpolation, bound, extrapolate)
     out = out.reshape(*batch, *outshape)
     if affine is not None:
         affine = torch.as_tensor(affine)

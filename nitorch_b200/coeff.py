@@ -39,7 +39,7 @@ def spline_coeff(inp, bound: int, order: int, dim: int = -1, inplace: bool = Fal
     if inp.numel() == 0:
         return out
     L = _lib.load()
-    with torch.cuda.device(inp.device):
+    with _lib.On(inp):
         _lib.check(L.pp_spline_coeff(ctypes.byref(_lib.desc(inp)), ctypes.byref(_lib.desc(out)),
                                      int(bound), int(order), int(dim), _lib.stream_of(inp)))
     return out
@@ -60,7 +60,7 @@ def spline_coeff_nd(inp, bound: List[int], order: List[int], dim: Optional[int] 
     B = (ctypes.c_int32 * len(b))(*b)
     O = (ctypes.c_int32 * len(o))(*o)
     L = _lib.load()
-    with torch.cuda.device(inp.device):
+    with _lib.On(inp):
         _lib.check(L.pp_spline_coeff_nd(ctypes.byref(_lib.desc(inp)), ctypes.byref(_lib.desc(out)),
                                         len(b), B, len(o), O, int(dim), _lib.stream_of(inp)))
     return out

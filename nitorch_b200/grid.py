@@ -9,6 +9,8 @@ saved tensors and backward unpacking by ``needs_input_grad``
 ``spatial.*_backward``: pull's input gradient is the push kernel and its
 grid gradient the fused derivative gather, both in one launch.
 """
+import functools
+
 import torch
 
 from . import coeff as _coeff
@@ -92,10 +94,18 @@ def inter_to_nitorch(inter, as_type="str"):
     return ointer
 
 
+@functools.lru_cache(maxsize=256)
+def _enums(bound, interpolation):
+    return (bound_to_nitorch(bound, as_type="enum"), inter_to_nitorch(interpolation, as_type="enum"))
+
+
 def _opt(bound, interpolation, extrapolate):
-    bound = bound_to_nitorch(make_list(bound), as_type="enum")
-    interpolation = inter_to_nitorch(make_list(interpolation), as_type="enum")
-    return bound, interpolation, int(extrapolate)
+    bound, interpolation = tuple(make_list(bound)), tuple(make_list(interpolation))
+    try:
+        bound, interpolation = _enums(bound, interpolation)
+    except TypeError:  # unhashable entries
+        bound, interpolation = _enums.__wrapped__(bound, interpolation)
+    return list(bound), list(interpolation), int(extrapolate)
 
 
 def _unpack(ctx, grads):

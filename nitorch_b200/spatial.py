@@ -291,23 +291,7 @@ def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, dtype=Non
     return o
 
 
-class _On:
-    """Make `t`'s device current for the duration of a launch."""
-    __slots__ = ("dev", "prev")
-
-    def __init__(self, t):
-        self.dev = t.device.index
-        self.prev = None
-
-    def __enter__(self):
-        cur = torch.cuda.current_device()
-        if self.dev is not None and cur != self.dev:
-            self.prev = cur
-            torch.cuda.set_device(self.dev)
-
-    def __exit__(self, *exc):
-        if self.prev is not None:
-            torch.cuda.set_device(self.prev)
+_On = _lib.On
 
 
 def _workspace(out):

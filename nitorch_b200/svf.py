@@ -22,17 +22,15 @@ import ctypes
 import torch
 
 from . import _lib
-from .grid import bound_to_nitorch, inter_to_nitorch
+from .grid import _opt
 from .spatial import _On, _require_cuda, get_deterministic
 
 __all__ = ["exp", "compose", "compose_backward"]
 
 
 def _options(interpolation, bound, extrapolate=True, flags=0):
-    b = bound_to_nitorch(bound if isinstance(bound, (list, tuple)) else [bound], as_type="enum")
-    o = inter_to_nitorch(interpolation if isinstance(interpolation, (list, tuple)) else [interpolation],
-                         as_type="enum")
-    return _lib.options([int(x) for x in b], [int(x) for x in o], int(extrapolate), flags)
+    b, o, extrapolate = _opt(bound, interpolation, extrapolate)
+    return _lib.options(b, o, extrapolate, flags)
 
 
 def _batched(field):
