@@ -197,8 +197,9 @@ class PullPushBatch:
         ref = lambda t: ctypes.byref(B.desc(t))  # noqa: E731
         opts = []
         for i in range(self.n):
-            # linear volumes run the direct kernels, in the grid's own order
-            if self.sorted_order and (self.orders[i] != 1 or self.flags):
+            # linear and one-channel quadratic volumes run the direct kernels, in the grid's own order
+            direct = not self.flags and (self.orders[i] == 1 or self.orders[i] == 2 and self.channels[i] == 1)
+            if self.sorted_order and not direct:
                 src = (ctypes.c_int64 * 3)(*self.shapes[i])
                 B.check(L.pp_brick_order(ref(self.grid[i]), src, ctypes.c_void_p(self.perm[i].data_ptr()),
                                          ctypes.c_void_p(self.starts[i].data_ptr()),

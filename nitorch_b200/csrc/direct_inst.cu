@@ -10,8 +10,8 @@
 
 cudaError_t PD_NAME(int ord, const ppk::PPArgs& a, cudaStream_t st) {
   if (ord == 1) return ppk::launch_direct_cb<PD_DIM, 1, PD_STYPE, PD_MODE>(a, st);
-#if PD_DIM == 2
   if (ord == 2) return ppk::launch_direct_cb<PD_DIM, 2, PD_STYPE, PD_MODE>(a, st);
+#if PD_DIM == 2
   if (ord == 3) return ppk::launch_direct_cb<PD_DIM, 3, PD_STYPE, PD_MODE>(a, st);
 #endif
   return cudaErrorInvalidValue;

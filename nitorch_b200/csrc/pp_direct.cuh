@@ -1,5 +1,6 @@
 // Direct kernels: sampling in the grid's own order for stencils of few taps
-// (3-D linear; 2-D linear, quadratic and cubic), float arithmetic.
+// (3-D linear, and quadratic where no brick order is given; 2-D linear,
+// quadratic and cubic), float arithmetic.
 //
 // The per-point kernel (pp_kernel) serves every order, bound, stride width
 // and flag; its index arithmetic -- 64-bit strides, per-tap offsets and
@@ -106,7 +107,7 @@ __device__ __forceinline__ void dir_axis(DirAxis<ORD + 1>& ax, int bnd, float x,
 // Resident CTAs of 256 threads the register budget is set for.
 template <int D, int ORD, int MODE, int CB> struct DirBlocks {
   static constexpr bool one = MODE == K_PULL || MODE == K_PUSH || MODE == K_COUNT;
-  static constexpr int value = D == 2 && ORD > 1 ? (one ? 3 : 2) : one ? (CB == 1 ? 5 : 4) : (CB == 1 ? 4 : 3);
+  static constexpr int value = ORD > 1 ? (one ? 3 : 2) : one ? (CB == 1 ? 5 : 4) : (CB == 1 ? 4 : 3);
 };
 
 // MODE as in pp_kernel: K_PULL, K_SGRAD, K_PUSH, K_COUNT, K_PULLGRAD,

@@ -1,5 +1,5 @@
-"""The direct kernels (3-D linear, 2-D linear to cubic, in the grid's own
-order) against the FP64 oracle where their tiling can go wrong: last axes of
+"""The direct kernels (3-D linear and quadratic, 2-D linear to cubic, in the
+grid's own order) against the FP64 oracle where their tiling can go wrong: last axes of
 one voxel, shorter and longer than a tile by one, ragged middle axes, runs of
 planes that end inside and across batch items, channel counts above a block,
 strided and broadcast tensors.  Tolerance: float32 arithmetic 1e-5, bfloat16
@@ -74,6 +74,12 @@ def _check(vol, grid, tgt, bound, order, ex, dtype=torch.float32, tol=1e-5):
 @pytest.mark.parametrize("bound,ex", [(7, 0), (2, 1), (3, 1)])
 def test_linear_3d_tile_edges(lattice, C, bound, ex):
     _check(*_case(lattice, (6, 7, 11), C, 2, C + sum(lattice)), bound, 1, ex)
+
+
+@pytest.mark.parametrize("lattice", SHAPES_3D)
+@pytest.mark.parametrize("bound,ex", [(7, 0), (2, 1), (3, 1)])
+def test_quadratic_3d_tile_edges(lattice, bound, ex):
+    _check(*_case(lattice, (6, 7, 11), 1, 2, 2 + sum(lattice)), bound, 2, ex)
 
 
 @pytest.mark.parametrize("lattice", SHAPES_2D)
