@@ -5,25 +5,24 @@
 // causal and one anti-causal first-order recursion per pole (coeff.py:
 // 254-281), initial / final conditions per boundary (coeff.py:69-251).
 //
-// B200 mapping: one line per thread, a tile of lines per CTA staged in
-// shared memory (element-major: warps of recursing threads read one sample of
-// 32 adjacent lines per access) by asynchronous copies issued for the whole
-// tile at once, 16 bytes at a time across adjacent lines when the filtered
-// axis is strided.  The sequential recursions run out of shared memory and
-// the global traffic is one read and one write of the volume per axis.  Tile
-// widths are chosen per line length so that two CTAs share an SM, one's
-// transfers overlapping the other's recursions.  The recursions run in float
-// (double for double storage); the initial / final condition sums in double
-// with per-pole constants computed on the host.  Lines too long for a shared
-// tile fall back to the same recursion directly on global memory.
+// B200 mapping: a tile of lines per CTA staged in shared memory (element-major:
+// warps of recursing threads read one sample of 32 adjacent lines per access),
+// the whole tile in flight at once, 16 bytes per access.  A line is cut into
+// segments, one thread each, whose recursions warm up over the end of the
+// neighbour: the poles forget within a few dozen samples.  The recursions run
+// out of shared memory and the global traffic is one read and one write of the
+// volume per axis; two or three CTAs share an SM, one's transfers overlapping
+// the others' recursions.  The recursions run in float (double for double
+// storage, whose lines stay whole); the initial / final condition sums in
+// double with per-pole constants computed on the host.  Lines too long for a
+// shared tile fall back to the same recursion directly on global memory.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "pp_capi_internal.cuh"
 
 namespace {
-
-constexpr int UNROLL = 8;     // 16-bit storage: loads in flight per thread while staging
 
 struct LineArgs {
   const void* in;
@@ -44,6 +43,9 @@ struct LineArgs {
   double zp[3];       // dct2: z^n; dct1: z^(n-1); dft: z^hz
   double zq[3];       // dct2: z^(2n-1-k2), k2 = max(1, 2n-1-K): the mirrored tail's first weight
   int line_major;     // 1: the filtered axis is the fastest (warps stage whole lines)
+  int quad_in, quad_out;  // line_major: all lines whole, aligned groups of four samples
+  int nseg;           // tile kernel: segments per line, one thread each
+  int warm;           // samples of a segment's warm-up: |z|^warm < 1e-13 for every pole
 };
 
 __device__ __forceinline__ void line_base(const LineArgs& a, int64_t l, int64_t& bi, int64_t& bo) {
@@ -57,284 +59,197 @@ __device__ __forceinline__ void line_base(const LineArgs& a, int64_t l, int64_t&
   }
 }
 
-// Accessors over V adjacent lines (V = 1: one line); load / store move
-// sample i of the V lines.
+// Accessors to the samples of one line.
 template <class C>
-struct LineRef {  // one line in global memory, any stride
-  static constexpr int V = 1;
+struct LineRef {  // in global memory, any stride
   using value_type = C;
   using index_type = int64_t;
   C* p;
   int64_t st;
-  __device__ __forceinline__ void load(int64_t i, C (&x)[1]) const { x[0] = p[i * st]; }
-  __device__ __forceinline__ void store(int64_t i, const C (&x)[1]) const { p[i * st] = x[0]; }
+  __device__ __forceinline__ C load(int64_t i) const { return p[i * st]; }
+  __device__ __forceinline__ void store(int64_t i, C x) const { p[i * st] = x; }
 };
 
 template <class C>
 struct TileLine {  // one column of a shared tile, runtime pitch
-  static constexpr int V = 1;
   using value_type = C;
   using index_type = int;
   C* p;
   int pitch;
-  __device__ __forceinline__ void load(int i, C (&x)[1]) const { x[0] = p[i * pitch]; }
-  __device__ __forceinline__ void store(int i, const C (&x)[1]) const { p[i * pitch] = x[0]; }
+  __device__ __forceinline__ C load(int i) const { return p[i * pitch]; }
+  __device__ __forceinline__ void store(int i, C x) const { p[i * pitch] = x; }
 };
 
-template <class C, int P, int V_>
-struct TileCols {  // V_ adjacent columns of a shared tile (compile-time pitch), one access
-  static constexpr int V = V_;
+template <class C, int P>
+struct TileCol {  // one column of a shared tile, compile-time pitch
   using value_type = C;
   using index_type = int;
   C* p;
-  __device__ __forceinline__ void load(int i, C (&x)[V]) const {
-    const C* q = p + i * P;
-    if constexpr (V == 4 && sizeof(C) == 4) {
-      const float4 t = *reinterpret_cast<const float4*>(q);
-      x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
-    } else if constexpr (V == 2 && sizeof(C) == 4) {
-      const float2 t = *reinterpret_cast<const float2*>(q);
-      x[0] = t.x; x[1] = t.y;
-    } else if constexpr (V == 2 && sizeof(C) == 8) {
-      const double2 t = *reinterpret_cast<const double2*>(q);
-      x[0] = t.x; x[1] = t.y;
-    } else {
-#pragma unroll
-      for (int c = 0; c < V; ++c) x[c] = q[c];
-    }
-  }
-  __device__ __forceinline__ void store(int i, const C (&x)[V]) const {
-    C* q = p + i * P;
-    if constexpr (V == 4 && sizeof(C) == 4) {
-      *reinterpret_cast<float4*>(q) = make_float4(x[0], x[1], x[2], x[3]);
-    } else if constexpr (V == 2 && sizeof(C) == 4) {
-      *reinterpret_cast<float2*>(q) = make_float2(x[0], x[1]);
-    } else if constexpr (V == 2 && sizeof(C) == 8) {
-      *reinterpret_cast<double2*>(q) = make_double2(x[0], x[1]);
-    } else {
-#pragma unroll
-      for (int c = 0; c < V; ++c) q[c] = x[c];
-    }
-  }
+  __device__ __forceinline__ C load(int i) const { return p[i * P]; }
+  __device__ __forceinline__ void store(int i, C x) const { p[i * P] = x; }
 };
 
-// Initial causal coefficient (coeff.py:69-170) of each of the V lines,
-// double accumulation.  The samples are read as L[k] * g (g: the filter gain
-// on the first pole's pass, 1 afterwards), so the gain costs no separate
-// sweep.
-template <class R, int V = R::V, class C = typename R::value_type>
-__device__ void initial(const R& L, int64_t n, const LineArgs& a, int q, C g, double (&out)[V]) {
+// Initial causal coefficient (coeff.py:69-170), double accumulation.  The
+// samples are read as L[k] * g (g: the filter gain on the first pole's pass,
+// 1 afterwards), so the gain costs no separate sweep.
+template <class R, class C = typename R::value_type>
+__device__ double initial(const R& L, int64_t n, const LineArgs& a, int q, C g) {
   const double z = a.z[q];
-  C t[V];
-  double xv[V], x0[V], acc[V];
-  auto x = [&](int64_t k) {
-    L.load(k, t);
-#pragma unroll
-    for (int c = 0; c < V; ++c) xv[c] = static_cast<double>(t[c] * g);
-  };
-  x(0);
-#pragma unroll
-  for (int c = 0; c < V; ++c) x0[c] = acc[c] = xv[c];
+  auto x = [&](int64_t k) { return static_cast<double>(L.load(static_cast<typename R::index_type>(k)) * g); };
+  const double x0 = x(0);
+  double acc = x0;
   if (a.kind == 2) {  // dct2 / replicate (coeff.py:137-170)
     const double zn = a.zp[q];
     const double zlast = zn * (1.0 + 1.0 / (z + zn * zn));
-    x(n - 1);
-#pragma unroll
-    for (int c = 0; c < V; ++c) acc[c] += zlast * xv[c];
+    acc += zlast * x(n - 1);
     // sum_{k=1}^{n-2} (z^k + z^(2n-1-k)) L[k]; both power series decay
     // geometrically, terms below 2^-64 of the leading one are dropped.
     const int64_t K = a.hz[q];
     const int64_t k1 = n - 2 < K ? n - 2 : K;
     double zk = z;
-    for (int64_t k = 1; k <= k1; ++k, zk *= z) {
-      x(k);
-#pragma unroll
-      for (int c = 0; c < V; ++c) acc[c] += zk * xv[c];
-    }
+    for (int64_t k = 1; k <= k1; ++k, zk *= z) acc += zk * x(k);
     int64_t k2 = 2 * n - 1 - K;
     if (k2 < 1) k2 = 1;
     if (k2 <= n - 2) {
       double zq = a.zq[q];
       const double iz = 1.0 / z;
-      for (int64_t k = k2; k <= n - 2; ++k, zq *= iz) {
-        x(k);
-#pragma unroll
-        for (int c = 0; c < V; ++c) acc[c] += zq * xv[c];
-      }
+      for (int64_t k = k2; k <= n - 2; ++k, zq *= iz) acc += zq * x(k);
     }
     const double s = z / (1.0 - zn * zn);
-#pragma unroll
-    for (int c = 0; c < V; ++c) out[c] = acc[c] * s + x0[c];
-    return;
+    return acc * s + x0;
   }
   if (a.kind == 1) {  // dct1 / zero (coeff.py:94-134)
     const int64_t m = a.hz[q];
     if (m < n) {
       double zk = z;
-      for (int64_t k = 1; k < m; ++k, zk *= z) {
-        x(k);
-#pragma unroll
-        for (int c = 0; c < V; ++c) acc[c] += zk * xv[c];
-      }
-#pragma unroll
-      for (int c = 0; c < V; ++c) out[c] = acc[c];
-      return;
+      for (int64_t k = 1; k < m; ++k, zk *= z) acc += zk * x(k);
+      return acc;
     }
     const double zn = a.zp[q];
-    x(n - 1);
-#pragma unroll
-    for (int c = 0; c < V; ++c) acc[c] += zn * xv[c];
+    acc += zn * x(n - 1);
     double zk = z;
-    for (int64_t k = 1; k < n - 1; ++k, zk *= z) {
-      x(k);
-      const double w = zk + zn * zn / zk;
-#pragma unroll
-      for (int c = 0; c < V; ++c) acc[c] += w * xv[c];
-    }
-    const double s = 1.0 / (1.0 - zn * zn);
-#pragma unroll
-    for (int c = 0; c < V; ++c) out[c] = acc[c] * s;
-    return;
+    for (int64_t k = 1; k < n - 1; ++k, zk *= z) acc += (zk + zn * zn / zk) * x(k);
+    return acc * (1.0 / (1.0 - zn * zn));
   }
   // dft (coeff.py:69-91)
   const int64_t m = a.hz[q];
   double zj = z;
-  for (int64_t j = 1; j < m; ++j, zj *= z) {
-    x(n - j);
-#pragma unroll
-    for (int c = 0; c < V; ++c) acc[c] += zj * xv[c];
-  }
-  const double s = 1.0 / (1.0 - a.zp[q]);
-#pragma unroll
-  for (int c = 0; c < V; ++c) out[c] = acc[c] * s;
+  for (int64_t j = 1; j < m; ++j, zj *= z) acc += zj * x(n - j);
+  return acc * (1.0 / (1.0 - a.zp[q]));
 }
 
-// Final anti-causal coefficient (coeff.py:173-215) of each of the V lines.
-template <class R, int V = R::V, class C = typename R::value_type>
-__device__ void final_value(const R& L, int64_t n, const LineArgs& a, int q, double (&out)[V]) {
+// Final anti-causal coefficient (coeff.py:173-215).
+template <class R>
+__device__ double final_value(const R& L, int64_t n, const LineArgs& a, int q) {
   const double z = a.z[q];
-  C t[V];
-  L.load(n - 1, t);
-  if (a.kind == 2) {
-    const double s = z / (z - 1.0);
-#pragma unroll
-    for (int c = 0; c < V; ++c) out[c] = static_cast<double>(t[c]) * s;
-    return;
-  }
-  if (a.kind == 1) {
-    C u[V];
-    L.load(n - 2, u);
-    const double s = z / (z * z - 1.0);
-#pragma unroll
-    for (int c = 0; c < V; ++c) out[c] = (z * static_cast<double>(u[c]) + static_cast<double>(t[c])) * s;
-    return;
-  }
+  auto x = [&](int64_t k) { return static_cast<double>(L.load(static_cast<typename R::index_type>(k))); };
+  if (a.kind == 2) return x(n - 1) * (z / (z - 1.0));
+  if (a.kind == 1) return (z * x(n - 2) + x(n - 1)) * (z / (z * z - 1.0));
   const int64_t m = a.hz[q];
-  double acc[V];
-#pragma unroll
-  for (int c = 0; c < V; ++c) acc[c] = z * static_cast<double>(t[c]);
+  double acc = z * x(n - 1);
   double zj = z * z;
-  for (int64_t j = 0; j < m - 1; ++j, zj *= z) {
-    L.load(j, t);
+  for (int64_t j = 0; j < m - 1; ++j, zj *= z) acc += zj * x(j);
+  return acc * (1.0 / (a.zp[q] - 1.0));
+}
+
+// One first-order recursion over `count` samples from i on, step DIR:
+//   causal       (DIR = 1):   c[i] = z c[i - 1] + g x[i]
+//   anti-causal  (DIR = -1):  c[i] = z (c[i + 1] - x[i])
+// `prev` enters as the coefficient before the first sample and leaves as the
+// last one.  The walk goes in chunks of U samples held in registers, the next
+// chunk loaded before the current one is filtered, so that the memory latency
+// leaves the dependency chain.  STORE = false only advances `prev`.
+template <int DIR, bool STORE, class R>
+__device__ __forceinline__ void walk(const R& L, typename R::index_type i, typename R::index_type count,
+                                     typename R::value_type z, typename R::value_type g,
+                                     typename R::value_type& prev) {
+  using C = typename R::value_type;
+  constexpr int U = 8;
+  auto step = [&](C x) { prev = DIR > 0 ? fma(z, prev, x * g) : z * (prev - x); };
+  if (count >= U) {
+    C x[U], y[U];
 #pragma unroll
-    for (int c = 0; c < V; ++c) acc[c] += zj * static_cast<double>(t[c]);
+    for (int u = 0; u < U; ++u) x[u] = L.load(i + DIR * u);
+    for (;;) {
+      const bool more = count >= 2 * U;
+      if (more) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) y[u] = L.load(i + DIR * (U + u));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        step(x[u]);
+        if (STORE) L.store(i + DIR * u, prev);
+      }
+      i += DIR * U;
+      count -= U;
+      if (!more) break;
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = y[u];
+    }
   }
-  const double s = 1.0 / (a.zp[q] - 1.0);
-#pragma unroll
-  for (int c = 0; c < V; ++c) out[c] = acc[c] * s;
+  for (; count > 0; --count, i += DIR) {
+    step(L.load(i));
+    if (STORE) L.store(i, prev);
+  }
 }
 
 // Gain (coeff.py:61-65) folded into the first causal pass, then one causal
-// and one anti-causal recursion per pole (coeff.py:254-281), on V lines at
-// once (independent dependency chains).  The walks go in chunks of U samples
-// held in registers, the next chunk loaded before the current one is
-// filtered, so that the memory latency leaves the dependency chains.
+// and one anti-causal recursion per pole (coeff.py:254-281).
 template <class R>
 __device__ void filter_line(const R& L, typename R::index_type n, const LineArgs& a) {
   using C = typename R::value_type;
-  using I = typename R::index_type;
-  constexpr int V = R::V;
-  constexpr int U = V == 1 ? 8 : 4;
   C g = static_cast<C>(a.gain);
   for (int q = 0; q < a.npoles; ++q) {
     const C z = static_cast<C>(a.z[q]);
-    double d[V];
-    C prev[V];
-    initial(L, n, a, q, g, d);
-#pragma unroll
-    for (int c = 0; c < V; ++c) prev[c] = static_cast<C>(d[c]);
+    C prev = static_cast<C>(initial(L, n, a, q, g));
     L.store(0, prev);
-    I i = 1;  // causal: i = 1 .. n-1
-    if (n - 1 >= U) {
-      C x[U][V];
-#pragma unroll
-      for (int u = 0; u < U; ++u) L.load(i + u, x[u]);
-      for (;;) {
-        const bool more = i + 2 * U <= n;
-        C y[U][V];
-        if (more) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) L.load(i + U + u, y[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-#pragma unroll
-          for (int c = 0; c < V; ++c) prev[c] = fma(z, prev[c], x[u][c] * g);
-          L.store(i + u, prev);
-        }
-        i += U;
-        if (!more) break;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int c = 0; c < V; ++c) x[u][c] = y[u][c];
-      }
-    }
-    for (; i < n; ++i) {
-      C x[V];
-      L.load(i, x);
-#pragma unroll
-      for (int c = 0; c < V; ++c) prev[c] = fma(z, prev[c], x[c] * g);
-      L.store(i, prev);
-    }
-    final_value(L, n, a, q, d);
-#pragma unroll
-    for (int c = 0; c < V; ++c) prev[c] = static_cast<C>(d[c]);
+    walk<1, true>(L, 1, n - 1, z, g, prev);
+    prev = static_cast<C>(final_value(L, n, a, q));
     L.store(n - 1, prev);
-    i = n - 2;  // anti-causal: i = n-2 .. 0
-    if (i + 1 >= U) {
-      C x[U][V];
-#pragma unroll
-      for (int u = 0; u < U; ++u) L.load(i - u, x[u]);
-      for (;;) {
-        const bool more = i + 1 >= 2 * U;
-        C y[U][V];
-        if (more) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) L.load(i - U - u, y[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-#pragma unroll
-          for (int c = 0; c < V; ++c) prev[c] = z * (prev[c] - x[u][c]);
-          L.store(i - u, prev);
-        }
-        i -= U;
-        if (!more) break;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int c = 0; c < V; ++c) x[u][c] = y[u][c];
-      }
+    walk<-1, true>(L, n - 2, n - 1, z, g, prev);
+    g = C(1);
+  }
+}
+
+// The same with the line cut into nseg segments, one thread of the CTA each
+// (thread (line, j) calls with its j; active: the thread has a line).  A
+// segment's recursion starts from a warm-up over the a.warm samples before
+// it, from zero: what is neglected is |z|^warm < 1e-13 of a coefficient,
+// far below the rounding of the float results.  The warm-ups read what the
+// neighbour is about to overwrite, hence the barriers; all threads of the CTA
+// make the call.
+template <class R>
+__device__ void filter_segment(const R& L, int n, const LineArgs& a, int j, bool active) {
+  using C = typename R::value_type;
+  const bool last = j == a.nseg - 1;
+  const int s = j * n / a.nseg, e = (j + 1) * n / a.nseg, w = a.warm;
+  C g = static_cast<C>(a.gain);
+  for (int q = 0; q < a.npoles; ++q) {
+    const C z = static_cast<C>(a.z[q]);
+    C prev = 0;
+    if (active) {
+      if (j == 0) prev = static_cast<C>(initial(L, n, a, q, g));
+      else walk<1, false>(L, s - w, w, z, g, prev);
     }
-    for (; i >= 0; --i) {
-      C x[V];
-      L.load(i, x);
-#pragma unroll
-      for (int c = 0; c < V; ++c) prev[c] = z * (prev[c] - x[c]);
-      L.store(i, prev);
+    __syncthreads();
+    if (active) {
+      if (j == 0) L.store(0, prev);
+      walk<1, true>(L, j == 0 ? 1 : s, e - (j == 0 ? 1 : s), z, g, prev);
+    }
+    __syncthreads();
+    prev = 0;
+    if (active) {
+      if (last) prev = static_cast<C>(final_value(L, n, a, q));
+      else walk<-1, false>(L, e + w - 1, w, z, g, prev);
+    }
+    __syncthreads();
+    if (active) {
+      if (last) L.store(n - 1, prev);
+      walk<-1, true>(L, last ? n - 2 : e - 1, (last ? n - 1 : e) - s, z, g, prev);
     }
     g = C(1);
+    __syncthreads();
   }
 }
 
@@ -370,37 +285,56 @@ __device__ __forceinline__ bool group_vec(const int64_t* base, const void* ptr, 
   return (p % bytes) == 0 && ((st * static_cast<int64_t>(sizeof(S))) % bytes) == 0;
 }
 
-// Full-tile kernel: NT lines per CTA (32, 64, 96 or 128: the widest that
-// leaves room for two CTAs per SM and one's transfers overlap the
-// other's recursions), held element-major in shared memory: tile[i * P + l],
-// P = NT + 4 (16-byte rows; 4 mod 32 words).  TILE_THREADS stage and store;
-// NT / V threads run the recursions, V adjacent lines each, read and written
-// as one access.  Staging keeps warps on consecutive global addresses:
-//  * filtered axis the fastest (line_major): a warp instruction covers 8
-//    consecutive samples of 4 lines (32-byte segments); with P = 4 mod 32
-//    words the 32 shared-memory writes fall in 32 distinct banks;
+// Four adjacent samples of one line, moved as one access (16 bytes of float
+// storage, 8 of 16-bit storage).
+template <class S>
+struct alignas(4 * sizeof(S)) Quad {
+  S v[4];
+  using C = typename ppk::Acc<S>::type;
+  using Raw = typename std::conditional<sizeof(S) == 2, uint2, uint4>::type;
+  __device__ __forceinline__ void load(const S* p) { *reinterpret_cast<Raw*>(this) = *reinterpret_cast<const Raw*>(p); }
+  __device__ __forceinline__ void store(S* p) const { *reinterpret_cast<Raw*>(p) = *reinterpret_cast<const Raw*>(this); }
+  __device__ __forceinline__ C get(int k) const { return ppk::to_acc(v[k]); }
+  __device__ __forceinline__ void set(int k, C x) { v[k] = ppk::from_acc<S>(x); }
+};
+
+// Full-tile kernel: NT lines per CTA, held element-major in shared memory
+// (tile[i * P + l]), staged and stored by TILE_THREADS threads; each line is
+// filtered by a.nseg of them (filter_segment).  With one thread per line the
+// recursions, two dependent passes of n steps, took longer than the
+// transfers: at 64 lines per CTA and four segments of 64 samples (warm-ups of
+// 23) per line of 256, three CTAs per SM, a pass over 3 x 256^3 floats takes
+// 91 / 87 / 107 us (first / middle / last axis; 136 / 121 / 150 with one
+// thread per line and 96 lines per CTA), 62 us of it memory traffic at the
+// copy rate; 3 x 192^3 48 / 48 / 50 us (55 / 55 / 69).  More registers per
+// thread or a fourth CTA per SM gain nothing further.
+//  * filtered axis the fastest (LM): a warp instruction covers 8 groups of
+//    four consecutive samples of 4 lines (128-byte segments), through
+//    registers; with an odd pitch the transposed writes (bank 4 qj + qs) fall
+//    in 32 distinct banks.  Lines that are not aligned for it: 8 single
+//    samples of 4 lines, 8 lines apart for the same reason.  (double: single
+//    samples of adjacent lines, P = NT + 4.)
 //  * otherwise each thread a group of G = 16 / sizeof(C) adjacent lines on
 //    every few sample rows, moved as one 16-byte copy (8-byte load for 16-bit
 //    storage) when the lines are adjacent and aligned in memory, else G
-//    scalar copies.
-// float / double storage stage with asynchronous copies, the whole tile in
-// flight at once; 16-bit storage converts through registers.
+//    scalar copies; P = NT + 4 (16-byte rows).
+// Strided float / double lines and single samples stage with asynchronous
+// copies, the whole tile in flight at once; 16-bit storage converts through
+// registers.
 constexpr int TILE_THREADS = 256;
-// lines per recursion thread: 1, 2 and 4 (one 4-, 8- or 16-byte access per
-// sample) measured within noise of each other on 3 x 192^3 and 3 x 256^3
-// float volumes; one line per thread keeps the most warps in the recursions
-constexpr int TILE_V = 1;
 
-template <class S, int NT, int V>
-__global__ void __launch_bounds__(TILE_THREADS, 2) coeff_tile_kernel(LineArgs a) {
+template <class C> constexpr int tile_pitch(int nt, bool line_major) { return line_major && sizeof(C) == 4 ? nt + 1 : nt + 4; }
+
+template <class S, int NT, bool LM>
+__global__ void __launch_bounds__(TILE_THREADS, sizeof(S) == 8 ? 2 : 3) coeff_tile_kernel(LineArgs a) {
   using C = typename ppk::Acc<S>::type;
   constexpr int G = 16 / static_cast<int>(sizeof(C));
-  constexpr int P = NT + 4;
+  constexpr int P = tile_pitch<C>(NT, LM);
   constexpr int NW = TILE_THREADS / 32;
   constexpr int GPR = NT / G;                 // strided: groups per sample row
   constexpr int RS = TILE_THREADS / GPR;      // strided: rows per step (threads past RS * GPR idle)
   constexpr bool kAsync = sizeof(S) == sizeof(C);
-  static_assert(NT % 32 == 0 && NT % G == 0 && RS >= 1 && NT / V <= TILE_THREADS, "tile shape");
+  static_assert(NT % 32 == 0 && NT % G == 0 && RS >= 1 && NT <= TILE_THREADS, "tile shape");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
   const int64_t l0 = static_cast<int64_t>(blockIdx.x) * NT;
@@ -413,29 +347,43 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) coeff_tile_kernel(LineArgs a)
   const int n32 = static_cast<int>(a.n);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int qs = lane >> 3, qj = lane & 7;  // line_major: line in the quad, first sample
+  // line_major, single samples: the lane's line in step qd
+  auto single_line = [&](int qd) { return P % 2 ? (qd >> 3) * 32 + (qd & 7) + 8 * qs : qd * 4 + qs; };
+  const bool vin = sizeof(C) == 4 && a.quad_in, vout = sizeof(C) == 4 && a.quad_out;
   const int gl = threadIdx.x < RS * GPR ? (threadIdx.x % GPR) * G : NT;  // strided: group (NT: idle)
   const int r0 = threadIdx.x / GPR;                                       // strided: first row
-  if (a.line_major) {
-    for (int qd = warp; qd * 4 < nl; qd += NW) {
-      const int l = qd * 4 + qs;
-      if (l >= nl) continue;
-      const S* src = in + bin[l];
-      C* dst = sm + l;
-      if constexpr (kAsync) {
-        for (int i = qj; i < n32; i += 8) cp_async<sizeof(C)>(dst + i * P, src + i * a.in_st);
-      } else {
-        for (int i0 = qj; i0 < n32; i0 += 8 * UNROLL) {
-          C v[UNROLL];
+  if constexpr (LM) {
+    if (vin) {
+      // 8 groups of 4 samples of 4 lines per warp instruction, 8 of them in flight
+      for (int qd = warp; qd * 4 < nl; qd += NW) {
+        const int l = qd * 4 + qs;
+        if (l >= nl) continue;
+        const S* src = in + bin[l];
+        for (int i0 = 4 * qj; i0 < n32; i0 += 256) {
+          Quad<S> v[8];
 #pragma unroll
-          for (int u = 0; u < UNROLL; ++u) {
-            const int i = i0 + 8 * u;
-            v[u] = i < n32 ? ppk::to_acc(src[i * a.in_st]) : C(0);
-          }
+          for (int u = 0; u < 8; ++u)
+            if (i0 + 32 * u < n32) v[u].load(src + i0 + 32 * u);
 #pragma unroll
-          for (int u = 0; u < UNROLL; ++u) {
-            const int i = i0 + 8 * u;
-            if (i < n32) dst[i * P] = v[u];
+          for (int u = 0; u < 8; ++u) {
+            C* dst = sm + (i0 + 32 * u) * P + l;
+            if (i0 + 32 * u < n32) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) dst[k * P] = v[u].get(k);
+            }
           }
+        }
+      }
+    } else {
+      for (int qd = warp; qd < NT / 4; qd += NW) {
+        const int l = single_line(qd);
+        if (l >= nl) continue;
+        const S* src = in + bin[l];
+        C* dst = sm + l;
+        if constexpr (kAsync) {
+          for (int i = qj; i < n32; i += 8) cp_async<sizeof(C)>(dst + i * P, src + i * a.in_st);
+        } else {
+          for (int i = qj; i < n32; i += 8) dst[i * P] = ppk::to_acc(src[i * a.in_st]);
         }
       }
     }
@@ -458,16 +406,29 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) coeff_tile_kernel(LineArgs a)
   }
   if constexpr (kAsync) asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-  // columns past nl (last tile) hold stale shared memory: filtered, never stored
-  if (threadIdx.x * V < nl) filter_line(TileCols<C, P, V>{sm + threadIdx.x * V}, n32, a);
-  __syncthreads();
-  if (a.line_major) {
-    for (int qd = warp; qd * 4 < nl; qd += NW) {
-      const int l = qd * 4 + qs;
-      if (l >= nl) continue;
-      S* dst = out + bout[l];
-      const C* src = sm + l;
-      for (int i = qj; i < n32; i += 8) dst[i * a.out_st] = ppk::from_acc<S>(src[i * P]);
+  const int col = threadIdx.x % NT, seg = threadIdx.x / NT;
+  filter_segment(TileCol<C, P>{sm + col}, n32, a, seg, seg < a.nseg && col < nl);
+  if constexpr (LM) {
+    if (vout) {
+      for (int qd = warp; qd * 4 < nl; qd += NW) {
+        const int l = qd * 4 + qs;
+        if (l >= nl) continue;
+        S* dst = out + bout[l];
+        for (int i = 4 * qj; i < n32; i += 32) {
+          Quad<S> v;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v.set(k, sm[(i + k) * P + l]);
+          v.store(dst + i);
+        }
+      }
+    } else {
+      for (int qd = warp; qd < NT / 4; qd += NW) {
+        const int l = single_line(qd);
+        if (l >= nl) continue;
+        S* dst = out + bout[l];
+        const C* src = sm + l;
+        for (int i = qj; i < n32; i += 8) dst[i * a.out_st] = ppk::from_acc<S>(src[i * P]);
+      }
     }
   } else if (gl < nl) {
     const bool vec = group_vec<S, G>(bout, out, a.out_st, gl, nl);
@@ -652,9 +613,11 @@ int allow_smem(K k, size_t smem, size_t static_bytes) {
                          "prefilter smem attribute");
 }
 
-template <class S, int NT, int V>
-int launch_tile(const LineArgs& a, size_t smem, cudaStream_t st) {
-  auto k = coeff_tile_kernel<S, NT, V>;
+template <class S, int NT, bool LM>
+int launch_tile(const LineArgs& a, cudaStream_t st) {
+  using C = typename ppk::Acc<S>::type;
+  auto k = coeff_tile_kernel<S, NT, LM>;
+  const size_t smem = static_cast<size_t>(a.n) * tile_pitch<C>(NT, LM) * sizeof(C);
   if (int rc = allow_smem(k, smem, 2 * NT * sizeof(int64_t))) return rc;
   const int64_t blocks = (a.nlines + NT - 1) / NT;
   k<<<static_cast<unsigned>(blocks), TILE_THREADS, smem, st>>>(a);
@@ -662,14 +625,28 @@ int launch_tile(const LineArgs& a, size_t smem, cudaStream_t st) {
   return ppc::cuda_check(cudaGetLastError(), "prefilter launch");
 }
 
+template <class S, int NT>
+int launch_tile(const LineArgs& a, cudaStream_t st) {
+  return a.line_major ? launch_tile<S, NT, true>(a, st) : launch_tile<S, NT, false>(a, st);
+}
+
 template <class S>
-int launch_tiles(const LineArgs& a, int NT, size_t smem, cudaStream_t st) {
-  switch (NT) {
-    case 128: return launch_tile<S, 128, TILE_V>(a, smem, st);
-    case 96: return launch_tile<S, 96, TILE_V>(a, smem, st);
-    case 64: return launch_tile<S, 64, TILE_V>(a, smem, st);
-    default: return launch_tile<S, 32, TILE_V>(a, smem, st);
-  }
+int launch_tiles(const LineArgs& a, int NT, cudaStream_t st) {
+  if (NT == 128) return launch_tile<S, 128>(a, st);
+  if (NT == 96) return launch_tile<S, 96>(a, st);
+  if (NT == 64) return launch_tile<S, 64>(a, st);
+  return launch_tile<S, 32>(a, st);
+}
+
+// Whether every line starts on, and consists of, aligned groups of four.  A
+// thread keeps the groups of one line in flight: lines of fewer than 96
+// samples leave too few (4 x 400 x 400 lines of 40: 137 us so, 101 us by
+// asynchronous copies of single samples).
+bool quads(const LineArgs& a, const void* p, int64_t st, const int64_t* os, size_t elem) {
+  if (st != 1 || a.n < 96 || a.n % 4 != 0 || reinterpret_cast<uintptr_t>(p) % (4 * elem) != 0) return false;
+  for (int d = 0; d < a.ndo; ++d)
+    if (a.osz[d] > 1 && os[d] % 4 != 0) return false;
+  return true;
 }
 
 template <class S>
@@ -678,14 +655,21 @@ int run_axis(LineArgs& a, cudaStream_t st) {
   constexpr int G = 16 / static_cast<int>(sizeof(C));
   if (a.nlines == 0) return PP_OK;
   const size_t budget = 200 * 1024;
-  // full tiles: the widest NT (multiple of 32, at most 128) whose tile
-  // leaves room for two CTAs per SM
+  // Full tiles: the widest NT (multiple of 32) whose tile leaves room for two
+  // CTAs per SM, at most 64 lines where a line has four segments or more (all
+  // threads recurse; at 96 lines there is room for two segments: 134 against
+  // 92 us on 3 x 256^3, at 32 for eight: 117 us) and 128 where it has fewer
+  // (4 x 400 x 400 lines of 40: 137 us at 64 lines, 94 at 128).
   {
     const int64_t fit = static_cast<int64_t>(113 * 1024 / (static_cast<size_t>(a.n) * sizeof(C))) - 4;
-    const int NT = fit >= 128 ? 128 : fit >= 96 ? 96 : fit >= 64 ? 64 : fit >= 32 ? 32 : 0;
+    const int64_t most = sizeof(C) == 4 ? a.n / (a.warm + 1) : 1;  // segments, each longer than a warm-up
+    const int most_nt = most >= 4 ? 64 : 128;
+    const int NT = static_cast<int>(std::min<int64_t>(most_nt, fit / 32 * 32));
     if (NT > 0) {
-      const size_t smem = static_cast<size_t>(a.n) * (NT + 4) * sizeof(C);
-      return launch_tiles<S>(a, NT, smem, st);
+      a.nseg = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(TILE_THREADS / NT, most)));
+      a.quad_in = quads(a, a.in, a.in_st, a.ist, sizeof(S));
+      a.quad_out = quads(a, a.out, a.out_st, a.ost, sizeof(S));
+      return launch_tiles<S>(a, NT, st);
     }
   }
   // longer lines: fewer per CTA, one per thread
@@ -736,11 +720,14 @@ int coeff_axis(const pp_tensor* in, const pp_tensor* out, int bound, int order, 
                         "(only zero, replicate, dct1, dct2 and dft)", bound);
   if (a.n == 1) return copy_any(in, out, st);
   a.gain = 1.0;
+  a.nseg = 1;
+  a.warm = 0;
   for (int q = 0; q < a.npoles; ++q) {
     const double z = a.z[q];
     a.gain *= (1.0 - z) * (1.0 - 1.0 / z);
     // truncation of the causal initial sums (coeff.py:75, :100): |z|^m < 1e-13
     const int64_t m = static_cast<int64_t>(std::ceil(-30.0 / std::log(std::fabs(z))));
+    a.warm = std::max(a.warm, static_cast<int>(m));
     if (a.kind == 2) {
       const int64_t K = static_cast<int64_t>(std::ceil(-44.4 / std::log(std::fabs(z)))) + 1;
       const int64_t k2 = std::max<int64_t>(1, 2 * a.n - 1 - K);
