@@ -347,14 +347,18 @@ __device__ __forceinline__ SampleAt sample_at(const BrickArgs& b, int v, int n) 
 // slots, 3: planes).
 // ===========================================================================
 // The warp walks `cnt` recorded points one at a time.  Cubic: lane (i, j, kk)
-// adds taps (i, j, kk) and (i, j, kk + 2) of the 4x4x4 support into its
-// window; quadratic: 27 lanes one tap each of the 3x3x3 support.
-template <int ORD, int CP>
-__device__ __forceinline__ void scatter_recorded(float* acc, const float* rec, int cnt, int lane) {
+// has taps (i, j, kk) and (i, j, kk + 2) of the 4x4x4 support; quadratic: 27
+// lanes one tap each of the 3x3x3 support.  RUNS: points of the same support,
+// which follow one another in brick order, are summed in registers and added
+// to the window at the end of their run (`ends`: bit q set where point q ends
+// one); else every point is added at once.
+template <int ORD, int CP, bool RUNS>
+__device__ __forceinline__ void scatter_walk(float* acc, const float* rec, int cnt, unsigned ends, int lane) {
   using W = BrickWin;
   const int ti = ORD == 3 ? lane >> 3 : lane / 9, tj = ORD == 3 ? (lane >> 1) & 3 : lane / 3 % 3;
   const int tk = ORD == 3 ? lane & 1 : lane % 3;
   const int loff = ti * W::PX + tj * W::PY + tk;
+  float s[2][CP] = {};
   for (int q = 0; q < cnt; ++q, rec += BRK_REC) {
     const float4 tq = *reinterpret_cast<const float4*>(rec + 12);
     const float tt[4] = {tq.x, tq.y, tq.z, tq.w};
@@ -362,16 +366,43 @@ __device__ __forceinline__ void scatter_recorded(float* acc, const float* rec, i
 #pragma unroll
     for (int c = 0; c < CP; ++c) t[c] = tt[c];
     const int vox0 = __float_as_int(CP < 4 ? tq.w : rec[16]) + loff;
-    if constexpr (ORD == 3) {
-      const float wxy = rec[ti] * rec[4 + tj];
-      const float2 zp = *reinterpret_cast<const float2*>(rec + 8 + 2 * tk);  // (wz_k, wz_k+2)
-      win_axpy<CP>(acc, vox0, wxy * zp.x, t);
-      win_axpy<CP>(acc, vox0 + 2, wxy * zp.y, t);
+    const float wxy = rec[ti] * rec[4 + tj];
+    const float2 zp = ORD == 3 ? *reinterpret_cast<const float2*>(rec + 8 + 2 * tk)  // (wz_k, wz_k+2)
+                               : make_float2(rec[8 + tk], 0.f);
+    const float w0 = wxy * zp.x, w1 = wxy * zp.y;
+    const bool on = ORD == 3 || lane < 27;
+    if constexpr (RUNS) {
+#pragma unroll
+      for (int c = 0; c < CP; ++c) {
+        s[0][c] = fmaf(w0, t[c], s[0][c]);
+        if (ORD == 3) s[1][c] = fmaf(w1, t[c], s[1][c]);
+      }
+      if (ends >> q & 1) {
+        if (on) win_axpy<CP>(acc, vox0, 1.f, s[0]);
+        if (ORD == 3) win_axpy<CP>(acc, vox0 + 2, 1.f, s[1]);
+#pragma unroll
+        for (int c = 0; c < CP; ++c) s[0][c] = s[1][c] = 0.f;
+        __syncwarp();
+      }
     } else {
-      if (lane < 27) win_axpy<CP>(acc, vox0, rec[ti] * rec[4 + tj] * rec[8 + tk], t);
+      if (on) win_axpy<CP>(acc, vox0, w0, t);
+      if (ORD == 3) win_axpy<CP>(acc, vox0 + 2, w1, t);
+      __syncwarp();
     }
-    __syncwarp();
   }
+}
+
+// Sums runs first where a warp's points have enough of them: at one run per
+// point the walk with runs takes up to 7 % longer (smooth deformations), at
+// 0.63 runs per point (independent uniform positions) 9 % less: 3 x 192^3,
+// rough, 0.652 -> 0.596 ms.  It also rounds less often.
+template <int ORD, int CP>
+__device__ __forceinline__ void scatter_recorded(float* acc, const float* rec, int cnt, int lane) {
+  const int at = lane < cnt ? __float_as_int(rec[lane * BRK_REC + (CP < 4 ? 15 : 16)]) : -1;
+  const int next = __shfl_down_sync(0xffffffffu, at, 1);
+  const unsigned ends = __ballot_sync(0xffffffffu, lane < cnt && (lane + 1 >= cnt || next != at));
+  if (__popc(ends) * 8 <= cnt * 7) scatter_walk<ORD, CP, true>(acc, rec, cnt, ends, lane);
+  else scatter_walk<ORD, CP, false>(acc, rec, cnt, ends, lane);
 }
 
 // Six CTAs per SM (at most 85 registers): the shared-memory budget of
