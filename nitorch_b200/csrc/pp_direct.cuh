@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
                   for (int q = 0; q < CB; ++q) sd[q] = fmaf(ax.g[i], v[q], sd[q]);
                 }
                 if (MODE == K_PULLGRAD || MODE == K_PUSHGRAD) {
-                  float dot = t[0] * v[0];
+                  float dot = CB == 1 ? v[0] : t[0] * v[0];  // one channel: scaled after the sums
 #pragma unroll
                   for (int q = 1; q < CB; ++q) dot = fmaf(t[q], v[q], dot);
                   sw[0] = D == 3 ? fmaf(ax.w[i], dot, sw[0]) : dot;
@@ -327,7 +327,10 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
             if (do_a) vp[(c0 + q) * a.trgt_sC] = from_acc<S>(val[q]);
           }
         }
-        if (MODE == K_PULLGRAD || MODE == K_PUSHGRAD) { og[0] += gx[0]; og[1] += gy[0]; og[2] += gz[0]; }
+        if (MODE == K_PULLGRAD || MODE == K_PUSHGRAD) {
+          const float sc = CB == 1 ? t[0] : 1.f;
+          og[0] += sc * gx[0]; og[1] += sc * gy[0]; og[2] += sc * gz[0];
+        }
       }
       // ---- scatter: LN lanes take one point's taps along the last axis --------
       if (SCATTER && (MODE != K_PUSHGRAD || do_a)) {
