@@ -288,14 +288,7 @@ SCATTER_OPS = ("push_fwd", "pull_bwd", "pp_fwd", "pp_bwd")
 # reports after the op.  Push and pull backward include the copy of their
 # channel-interleaved accumulator into the output (store_interleaved_vox).
 # A kernel not listed here reports traffic null.
-MEASURED_TRAFFIC = {
-    "pp_brick_gather_kernel mode=0 order=3 cb=3": 291_602_176,
-    "pp_brick_scatter_kernel mode=2 order=3 cb=3": 413_647_360 + 152_769_792,
-    "pp_kernel mode=4 order=3 cb=3": 492_331_520,
-    "pp_brick_pullbwd_kernel mode=5 order=3 cb=3": 583_946_240 + 151_942_400,
-    # resize 1x3x256^3 -> 320^3, cubic, dct2
-    "resize_sep_kernel tma mode=0 order=3 cb=1": 566_675_200,
-}
+MEASURED_TRAFFIC = {}  # no capture of the kernels as they are now
 
 
 def roofline(ops, labels, nvox, C, ms_per_step, traffic):

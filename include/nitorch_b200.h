@@ -96,10 +96,11 @@ typedef struct pp_options {
   const int32_t* brick_start;    /* optional device array, 3-D grids only:
                                     with sample_order from pp_brick_order,
                                     its brick offsets (N * nbricks + 1
-                                    entries).  Lets the cubic scatters
-                                    accumulate each brick of the scatter
-                                    target in on-chip memory.  NULL = no
-                                    brick pass.                           */
+                                    entries).  Quadratic and cubic calls on
+                                    float32 / bfloat16 images of up to four
+                                    channels then hold each brick of the
+                                    source or scatter target in on-chip
+                                    memory.  NULL = no brick pass.        */
   const float* brick_records;    /* optional device array with brick_start:
                                     the records pp_brick_order wrote for
                                     the same float32 grid (4 floats per
@@ -121,7 +122,7 @@ PP_API const char* pp_last_error(void);
 PP_API unsigned long long pp_kernel_launches(void);
 
 /* Kernel family, mode, order and channel block of the last push/pull
- * launch made on this host thread, e.g. "pp_brick_kernel mode=5 order=3
+ * launch made on this host thread, e.g. "pp_brick_pullbwd_kernel mode=5 order=3
  * cb=3" ("" if none); for auditing which code path a call took. */
 PP_API const char* pp_last_kernel(void);
 
@@ -354,7 +355,7 @@ PP_API int pp_sample_order(const pp_tensor* grid, const int64_t* src_size, int32
                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* Brick-major processing order (no counterpart in the reference; a
- * scheduling aid for the cubic 3-D brick kernels).  The source volume (spatial
+ * scheduling aid for the 3-D brick kernels, quadratic and cubic).  The source volume (spatial
  * size `src_size`, 3 entries) is cut into bricks of PP_BRICK_X x PP_BRICK_Y
  * x PP_BRICK_Z voxels, nb = prod(ceil(src_size / brick)) per batch item.
  * Writes to `perm` (int32, N*prod(grid spatial) entries) the sample

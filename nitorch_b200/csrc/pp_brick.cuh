@@ -15,7 +15,8 @@
 //      out-of-bound test, B-spline weights), into shared records;
 //   3. the warp walks the recorded points one at a time, lane (i, j, kk)
 //      taking taps (i, j, kk) and (i, j, kk + 2) of a 4x4x4 support (27 lanes
-//      the taps of a 3x3x3 support): plain shared read-modify-writes (the
+//      the taps of a 3x3x3 support), runs of points of one support summed
+//      first where there are many: plain shared read-modify-writes (the
 //      lanes touch distinct voxels and the window belongs to this warp
 //      alone, so no atomics);
 //   4. the window is added to the output with one vector reduction per
@@ -41,11 +42,11 @@
 //
 // Measured on 3 x 192^3, cubic, rough deformation (std 4 over 2 voxels), one
 // brick per CTA (push backward: the per-point kernel) before and this form
-// after: pull 0.654 -> 0.462 ms, push backward 1.111 -> 0.725 ms, pull
-// backward (was one kernel for both gradients) 1.755 -> 0.723 + 0.655 ms, push
-// 0.731 -> 0.655 ms.  160 x 192 x 160, one channel: pull 0.322 -> 0.173 ms,
-// grid gradient 0.583 -> 0.286 ms.  The gathers are latency-bound (scattered
-// reads and writes by sample index, two or three CTAs per SM).
+// after: pull 0.654 -> 0.419 ms, push backward 1.111 -> 0.657 ms, pull
+// backward (was one kernel for both gradients) 1.755 -> 0.670 + 0.596 ms, push
+// 0.731 -> 0.596 ms.  160 x 192 x 160, one channel: pull 0.322 -> 0.171 ms,
+// grid gradient 0.583 -> 0.282 ms.  The gathers are latency-bound (scattered
+// reads and writes by sample index, three or four CTAs per SM).
 //
 // Points whose support leaves the window (sampling outside the volume with
 // extrapolation, or just below a volume edge) run the per-point body

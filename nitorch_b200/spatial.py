@@ -59,7 +59,8 @@ def set_sample_order(mode="auto"):
     """Processing order of the sampling points: "natural" (grid order),
     "sorted" (brick-major for 3-D grids, see pp_brick_order; source-sorted
     for 1-D / 2-D, see pp_sample_order) or "auto" (sorted for grids of at
-    least 2^18 points).  Only the speed depends on it."""
+    least 2^18 points, but for calls of the direct kernels).  Only the speed
+    depends on it."""
     global _sample_order_mode
     if mode not in ("auto", "natural", "sorted"):
         raise ValueError(f"unknown sample order mode {mode}")
