@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(256) brick_count(const BrickKeyArgs b, int32_t
 
 // The scatter pass: the scanned counts are cursors, advanced to their keys'
 // ends.  Each sample's key is formed again from the grid (12 bytes read; its
-// stored key and rank would be 8 bytes written and 8 read, and workspace).
+// stored key and rank would be 8 bytes written and 8 read; the workspace still
+// has room for them, as its callers may have sized it).
 // Count and scatter of 192^3 samples, smooth deformation: 42 + 125 us (65 + 117
 // with stored keys and ranks); 160^3, rough: 42 + 83 us (59 + 76).  Bound by
 // scattered 4- and 16-byte writes; four samples per thread, for more atomics
@@ -318,7 +319,7 @@ size_t pp_brick_order_workspace_bytes(const pp_tensor* grid, const int64_t* src_
   int64_t nvox;
   BrickGeom g;
   if (brick_sizes_of(grid, src_size, nvox, g)) return 0;
-  return layout(0, g.nkeys).total;
+  return layout(nvox, g.nkeys).total;
 }
 
 int pp_brick_order(const pp_tensor* grid, const int64_t* src_size, int32_t* perm, int32_t* brick_start,
@@ -330,7 +331,7 @@ int pp_brick_order(const pp_tensor* grid, const int64_t* src_size, int32_t* perm
   if (!perm || !brick_start) return ppc::fail(PP_ERR_ARG, "(): expected an output permutation and brick offsets");
   if (records && (grid->dtype != PP_FLOAT32 || reinterpret_cast<uintptr_t>(records) % 16 != 0))
     return ppc::fail(PP_ERR_ARG, "(): brick records need a float32 grid and a 16-byte aligned buffer");
-  const Layout L = layout(0, g.nkeys);
+  const Layout L = layout(nvox, g.nkeys);
   if (!workspace || workspace_bytes < L.total)
     return ppc::fail(PP_ERR_WORKSPACE, "(): brick ordering needs %zu bytes of workspace", L.total);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
