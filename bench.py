@@ -288,7 +288,12 @@ SCATTER_OPS = ("push_fwd", "pull_bwd", "pp_fwd", "pp_bwd")
 # reports after the op.  Push and pull backward include the copy of their
 # channel-interleaved accumulator into the output (store_interleaved_vox).
 # A kernel not listed here reports traffic null.
-MEASURED_TRAFFIC = {}  # no capture of the kernels as they are now
+MEASURED_TRAFFIC = {
+    "pp_brick_gather_kernel mode=0 order=3 cb=3": 289_696_256,
+    "pp_brick_scatter_kernel mode=2 order=3 cb=3": 399_176_192 + 146_609_152,
+    "pp_brick_gather_kernel mode=4 order=3 cb=3": 523_536_384,
+    "pp_brick_pullbwd_kernel mode=5 order=3 cb=3": 400_533_504 + 379_292_416 + 146_874_368,
+}
 
 
 def roofline(ops, labels, nvox, C, ms_per_step, traffic):

@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(256) brick_count(const BrickKeyArgs b, int32_t
 // ends.  Each sample's key is formed again from the grid (12 bytes read; its
 // stored key and rank would be 8 bytes written and 8 read; the workspace still
 // has room for them, as its callers may have sized it).
-// Count and scatter of 192^3 samples, smooth deformation: 42 + 125 us (65 + 117
-// with stored keys and ranks); 160^3, rough: 42 + 83 us (59 + 76).  Bound by
+// Count and scatter of 192^3 samples, rough deformation: 42 + 125 us (65 + 117
+// with stored keys and ranks); 181 x 217 x 181, smoother: 42 + 83 us (59 + 76).  Bound by
 // scattered 4- and 16-byte writes; four samples per thread, for more atomics
 // in flight, spread the writes further: 154 us.  With `rec`, the
 // sample's coordinates and index also go as one 16-byte record to its place,
