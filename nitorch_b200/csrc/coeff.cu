@@ -158,14 +158,26 @@ __device__ double final_value(const R& L, int64_t n, const LineArgs& a, int q) {
 // `prev` enters as the coefficient before the first sample and leaves as the
 // last one.  The walk goes in chunks of U samples held in registers, the next
 // chunk loaded before the current one is filtered, so that the memory latency
-// leaves the dependency chain.  STORE = false only advances `prev`.
+// leaves the dependency chain.  STORE = false only advances `prev`.  The
+// operations of a step are written out (diff = c[i + 1] - x[i], carried along the
+// anti-causal walk): contracted as the compiler likes, a warm-up and the walk
+// that it stands in for would round differently and never arrive at one value.
 template <int DIR, bool STORE, class R>
 __device__ __forceinline__ void walk(const R& L, typename R::index_type i, typename R::index_type count,
                                      typename R::value_type z, typename R::value_type g,
                                      typename R::value_type& prev) {
   using C = typename R::value_type;
   constexpr int U = 8;
-  auto step = [&](C x) { prev = DIR > 0 ? fma(z, prev, x * g) : z * (prev - x); };
+  C diff = prev, zz = 1;  // (the first difference is from `prev` itself)
+  auto step = [&](C x) {
+    if (DIR > 0) {
+      prev = fma(z, prev, x * g);
+    } else {
+      diff = fma(zz, diff, -x);
+      zz = z;
+      prev = z * diff;
+    }
+  };
   if (count >= U) {
     C x[U], y[U];
 #pragma unroll
@@ -212,13 +224,47 @@ __device__ void filter_line(const R& L, typename R::index_type n, const LineArgs
   }
 }
 
+// Two recursions are at the same value (two NaNs are).
+template <class C> __device__ __forceinline__ bool differ(C x, C y) { return !(x == y) && (x == x || y == y); }
+
+// Segments whose recursions began elsewhere than their neighbours' ended: the
+// difference runs on through the segment as d z, d z^2, ... (the recursions
+// are linear).  `count` samples from i on, step DIR; `has`: a neighbour ends
+// right before i; from: the segment's start.  A segment is right once those
+// before it are, hence nseg - 1 rounds at most.  All threads of the CTA.
+template <int DIR, class R>
+__device__ __noinline__ void settle(const R& L, int i, int count, bool has, typename R::value_type z,
+                                    typename R::value_type from, int nseg) {
+  using C = typename R::value_type;
+  for (int k = 1; k < nseg; ++k) {
+    const C end = has ? L.load(i - DIR) : from;
+    const bool off = differ(end, from);
+    if (!__syncthreads_or(off)) return;
+    if (off) {
+      C d = end - from;
+      for (int m = 0; m < count && d != C(0); ++m) {
+        d *= z;
+        L.store(i + DIR * m, L.load(i + DIR * m) + d);
+      }
+    }
+    from = end;
+    __syncthreads();
+  }
+}
+
 // The same with the line cut into nseg segments, one thread of the CTA each
 // (thread (line, j) calls with its j; active: the thread has a line).  A
 // segment's recursion starts from a warm-up over the a.warm samples before
-// it, from zero: what is neglected is |z|^warm < 1e-13 of a coefficient,
-// far below the rounding of the float results.  The warm-ups read what the
-// neighbour is about to overwrite, hence the barriers; all threads of the CTA
-// make the call.
+// it, from zero.  That is where the whole line's recursion would arrive, but
+// for what |z|^warm < 1e-13 leaves of the coefficients before the warm-up:
+// nothing in float between samples of like size, but everything next to an
+// infinity, a NaN or a sample 1e13 times as large.  So each segment then
+// compares its start with its neighbour's end, and where they differ (in the
+// lines of ordinary volumes only past a stretch of exact zeros) the difference
+// is carried on until all agree: the result is the whole line's.  (The checks
+// cost 2-4 %: 3 x 256^3 cubic 274 -> 280 us for the three axes, 3 x 192^3
+// 125 -> 128 us.)  The warm-ups read what the neighbour is about to overwrite,
+// hence the barriers; all threads of the CTA make the call.
 template <class R>
 __device__ void filter_segment(const R& L, int n, const LineArgs& a, int j, bool active) {
   using C = typename R::value_type;
@@ -232,24 +278,33 @@ __device__ void filter_segment(const R& L, int n, const LineArgs& a, int j, bool
       if (j == 0) prev = static_cast<C>(initial(L, n, a, q, g));
       else walk<1, false>(L, s - w, w, z, g, prev);
     }
+    C from = prev;
     __syncthreads();
     if (active) {
       if (j == 0) L.store(0, prev);
       walk<1, true>(L, j == 0 ? 1 : s, e - (j == 0 ? 1 : s), z, g, prev);
     }
     __syncthreads();
-    prev = 0;
-    if (active) {
-      if (last) prev = static_cast<C>(final_value(L, n, a, q));
-      else walk<-1, false>(L, e + w - 1, w, z, g, prev);
+    for (bool right = false;;) {
+      const bool off = !right && active && j > 0 && differ(L.load(s - 1), from);
+      prev = 0;
+      if (active) {
+        if (last) prev = static_cast<C>(final_value(L, n, a, q));
+        else walk<-1, false>(L, e + w - 1, w, z, g, prev);
+      }
+      if (!__syncthreads_or(off)) break;
+      settle<1>(L, s, e - s, active && j > 0, z, from, a.nseg);  // ... and the warm-up again
+      right = true;
     }
-    __syncthreads();
+    from = prev;
     if (active) {
       if (last) L.store(n - 1, prev);
       walk<-1, true>(L, last ? n - 2 : e - 1, (last ? n - 1 : e) - s, z, g, prev);
     }
     g = C(1);
     __syncthreads();
+    if (__syncthreads_or(active && !last && differ(L.load(e), from)))
+      settle<-1>(L, e - 1, e - s, active && !last, z, from, a.nseg);
   }
 }
 
@@ -407,7 +462,13 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(S) == 8 ? 2 : 3) coeff_ti
   if constexpr (kAsync) asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   const int col = threadIdx.x % NT, seg = threadIdx.x / NT;
-  filter_segment(TileCol<C, P>{sm + col}, n32, a, seg, seg < a.nseg && col < nl);
+  const bool active = seg < a.nseg && col < nl;
+  if (a.nseg > 1) {
+    filter_segment(TileCol<C, P>{sm + col}, n32, a, seg, active);
+  } else {
+    if (active) filter_line(TileCol<C, P>{sm + col}, n32, a);
+    __syncthreads();
+  }
   if constexpr (LM) {
     if (vout) {
       for (int qd = warp; qd * 4 < nl; qd += NW) {
@@ -662,8 +723,11 @@ int run_axis(LineArgs& a, cudaStream_t st) {
   // (4 x 400 x 400 lines of 40: 137 us at 64 lines, 94 at 128).
   {
     const int64_t fit = static_cast<int64_t>(113 * 1024 / (static_cast<size_t>(a.n) * sizeof(C))) - 4;
-    const int64_t most = sizeof(C) == 4 ? a.n / (a.warm + 1) : 1;  // segments, each longer than a warm-up
-    const int most_nt = most >= 4 ? 64 : 128;
+    // segments, each longer than a warm-up; with fewer than four their warm-ups
+    // and checks cost what they save (cubic 72^3: 20.3 us in two, 19.0 whole)
+    int64_t most = sizeof(C) == 4 ? a.n / (a.warm + 1) : 1;
+    if (most < 4) most = 1;
+    const int most_nt = most > 1 ? 64 : 128;
     const int NT = static_cast<int>(std::min<int64_t>(most_nt, fit / 32 * 32));
     if (NT > 0) {
       a.nseg = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(TILE_THREADS / NT, most)));
