@@ -112,7 +112,16 @@ template <int D, int ORD, int MODE, int CB> struct DirBlocks {
 
 // MODE as in pp_kernel: K_PULL, K_SGRAD, K_PUSH, K_COUNT, K_PULLGRAD,
 // K_PUSHGRAD; 1 << tzs points of a CTA's tile lie along the last axis.
-template <int D, int ORD, int CB, class S, int MODE>
+//
+// Grid gradient, sum_c t[c] sum_nodes dw src[c]: the nodes' differences first,
+// each channel's by itself, its product with t after them.  DOT: the products
+// of all channels first, one sum over the nodes of their dot product; fewer
+// registers, but the differences then carry the rounding of the products (rms
+// error of 2-D linear gradients of a smooth 4-channel image: 4.7e-7 against
+// 2.2e-7; 4 x 8 x 512^2 cubic, both passes: 301 and 308 us).  Only the
+// 3-D linear pull backward of two to four channels sums so, as its lane-split
+// kernel (pp_lanes_pullbwd_kernel) does.
+template <int D, int ORD, int CB, class S, int MODE, bool DOT>
 __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::value))
     pp_direct_kernel(const __grid_constant__ DirArgs a) {
   constexpr int NT = ORD + 1;
@@ -240,7 +249,7 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
       // ---- gather: separable sums, the first axis innermost ------------------
       if (GATHER && live && (MODE != K_PUSHGRAD || do_grad)) {
         const S* sp = sn + c0 * a.src_sC;
-        constexpr int NGC = MODE == K_SGRAD ? CB : 1;  // gradients per channel, or of the dot product with t
+        constexpr int NGC = DOT ? 1 : CB;  // gradients of the dot product with t, or per channel
         float val[CB], gx[NGC], gy[NGC], gz[NGC];
 #pragma unroll
         for (int q = 0; q < CB; ++q) val[q] = 0.f;
@@ -269,16 +278,14 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
                 float v[CB];
 #pragma unroll
                 for (int q = 0; q < CB; ++q) v[q] = (ok && (CB == 1 || q < nc)) ? ldg_acc(p + q * a.src_sC) : 0.f;
-                if (MODE != K_PUSHGRAD) {
+                if (!DOT) {
 #pragma unroll
-                  for (int q = 0; q < CB; ++q) sv[q] = D == 3 ? fmaf(ax.w[i], v[q], sv[q]) : v[q];
-                }
-                if (MODE == K_SGRAD && D == 3) {
-#pragma unroll
-                  for (int q = 0; q < CB; ++q) sd[q] = fmaf(ax.g[i], v[q], sd[q]);
-                }
-                if (MODE == K_PULLGRAD || MODE == K_PUSHGRAD) {
-                  float dot = CB == 1 ? v[0] : t[0] * v[0];  // one channel: scaled after the sums
+                  for (int q = 0; q < CB; ++q) {
+                    sv[q] = D == 3 ? fmaf(ax.w[i], v[q], sv[q]) : v[q];
+                    if (NEED_G && D == 3) sd[q] = fmaf(ax.g[i], v[q], sd[q]);
+                  }
+                } else {
+                  float dot = t[0] * v[0];
 #pragma unroll
                   for (int q = 1; q < CB; ++q) dot = fmaf(t[q], v[q], dot);
                   sw[0] = D == 3 ? fmaf(ax.w[i], dot, sw[0]) : dot;
@@ -287,12 +294,12 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
               }
 #pragma unroll
               for (int q = 0; q < CB; ++q)
-                if (MODE != K_PUSHGRAD) zv[q] = fmaf(ay.w[j], sv[q], zv[q]);
+                if (!DOT) zv[q] = fmaf(ay.w[j], sv[q], zv[q]);
               if (NEED_G) {
 #pragma unroll
                 for (int q = 0; q < NGC; ++q) {
-                  const float s0 = MODE == K_SGRAD ? sv[q] : sw[q];
-                  if (MODE != K_SGRAD) zw[q] = fmaf(ay.w[j], s0, zw[q]);
+                  const float s0 = DOT ? sw[q] : sv[q];
+                  if (DOT) zw[q] = fmaf(ay.w[j], s0, zw[q]);
                   if (D == 3) zgx[q] = fmaf(ay.w[j], sd[q], zgx[q]);
                   zgy[q] = fmaf(ay.g[j], s0, zgy[q]);
                 }
@@ -306,7 +313,7 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
               for (int q = 0; q < NGC; ++q) {
                 if (D == 3) gx[q] = fmaf(az.w[k], zgx[q], gx[q]);
                 gy[q] = fmaf(az.w[k], zgy[q], gy[q]);
-                gz[q] = fmaf(az.g[k], MODE == K_SGRAD ? zv[q] : zw[q], gz[q]);
+                gz[q] = fmaf(az.g[k], DOT ? zw[q] : zv[q], gz[q]);
               }
             }
           }
@@ -328,8 +335,11 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
           }
         }
         if (MODE == K_PULLGRAD || MODE == K_PUSHGRAD) {
-          const float sc = CB == 1 ? t[0] : 1.f;
-          og[0] += sc * gx[0]; og[1] += sc * gy[0]; og[2] += sc * gz[0];
+#pragma unroll
+          for (int q = 0; q < NGC; ++q) {
+            const float sc = DOT ? 1.f : t[q];
+            og[0] = fmaf(sc, gx[q], og[0]); og[1] = fmaf(sc, gy[q], og[1]); og[2] = fmaf(sc, gz[q], og[2]);
+          }
         }
       }
       // ---- scatter: LN lanes take one point's taps along the last axis --------
@@ -378,7 +388,7 @@ __global__ void __launch_bounds__(DIR_THREADS, (DirBlocks<D, ORD, MODE, CB>::val
   }
 }
 
-template <int D, int ORD, int CB, class S, int MODE>
+template <int D, int ORD, int CB, class S, int MODE, bool DOT = false>
 inline cudaError_t launch_direct(const PPArgs& p, cudaStream_t st) {
   DirArgs a;
   a.src = p.src; a.trgt = p.trgt; a.grid = static_cast<const float*>(p.grid);
@@ -426,7 +436,7 @@ inline cudaError_t launch_direct(const PPArgs& p, cudaStream_t st) {
   a.run = static_cast<int>(run);
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>((a.outer + run - 1) / run));
   note_kernel("pp_direct_kernel", MODE, ORD, CB);
-  pp_direct_kernel<D, ORD, CB, S, MODE><<<grid, DIR_THREADS, 0, st>>>(a);
+  pp_direct_kernel<D, ORD, CB, S, MODE, DOT><<<grid, DIR_THREADS, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -434,10 +444,13 @@ inline cudaError_t launch_direct(const PPArgs& p, cudaStream_t st) {
 template <int D, int ORD, class S, int MODE>
 inline cudaError_t launch_direct_cb(const PPArgs& a, cudaStream_t st) {
   if constexpr (MODE != K_COUNT) {
+    constexpr bool DOT = D == 3 && ORD == 1 && MODE == K_PUSHGRAD;
     switch (a.C >= 4 ? 4 : static_cast<int>(a.C)) {
-      case 2: return launch_direct<D, ORD, 2, S, MODE>(a, st);
-      case 3: return launch_direct<D, ORD, 3, S, MODE>(a, st);
-      case 4: return launch_direct<D, ORD, 4, S, MODE>(a, st);
+      case 2: return launch_direct<D, ORD, 2, S, MODE, DOT>(a, st);
+      case 3: return launch_direct<D, ORD, 3, S, MODE, DOT>(a, st);
+      case 4:
+        if (a.C > 4) return launch_direct<D, ORD, 4, S, MODE>(a, st);
+        return launch_direct<D, ORD, 4, S, MODE, DOT>(a, st);
       default: break;
     }
   }
