@@ -94,17 +94,20 @@ def inter_to_nitorch(inter, as_type="str"):
     return ointer
 
 
-@functools.lru_cache(maxsize=256)
 def _enums(bound, interpolation):
     return (bound_to_nitorch(bound, as_type="enum"), inter_to_nitorch(interpolation, as_type="enum"))
 
 
+_known_enums = functools.lru_cache(maxsize=256)(_enums)
+# entries that are equal for good; others (a tensor hashes by identity and can
+# change its value) are read anew on each call
+_CONSTANT = (str, int, BoundType, InterpolationType)
+
+
 def _opt(bound, interpolation, extrapolate):
     bound, interpolation = tuple(make_list(bound)), tuple(make_list(interpolation))
-    try:
-        bound, interpolation = _enums(bound, interpolation)
-    except TypeError:  # unhashable entries
-        bound, interpolation = _enums.__wrapped__(bound, interpolation)
+    constant = all(type(x) in _CONSTANT for x in bound + interpolation)
+    bound, interpolation = (_known_enums if constant else _enums)(bound, interpolation)
     return list(bound), list(interpolation), int(extrapolate)
 
 
