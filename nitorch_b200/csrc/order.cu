@@ -229,10 +229,11 @@ struct BrickKeyArgs {
   int nbx, nby, nbz;
 };
 
-// Coordinates of sample s and its key.
+// The coordinates of sample s in the grid; v: its batch item.
 template <class T>
-__device__ __forceinline__ int brick_key(const BrickKeyArgs& b, unsigned s, T (&c)[3]) {
-  unsigned v = s, sub[3];
+__device__ __forceinline__ const T* sample_ptr(const BrickKeyArgs& b, unsigned s, unsigned& v) {
+  unsigned sub[3];
+  v = s;
 #pragma unroll
   for (int d = 2; d >= 0; --d) {
     const unsigned n = static_cast<unsigned>(b.k.size[d]), q = v / n;
@@ -242,12 +243,20 @@ __device__ __forceinline__ int brick_key(const BrickKeyArgs& b, unsigned s, T (&
   const T* g = static_cast<const T*>(b.k.grid) + static_cast<int64_t>(v) * b.k.gsN;
 #pragma unroll
   for (int d = 0; d < 3; ++d) g += static_cast<int64_t>(sub[d]) * b.k.gs[d];
+  return g;
+}
+
+// Key of sample s.
+template <class T>
+__device__ __forceinline__ int brick_key(const BrickKeyArgs& b, unsigned s) {
+  unsigned v;
+  const T* g = sample_ptr<T>(b, s, v);
   int f[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    c[d] = g[d * b.k.gsD];
+    const T c = g[d * b.k.gsD];
     const int n = static_cast<int>(b.k.src[d]);
-    f[d] = (c[d] >= T(0)) ? static_cast<int>(fmin(c[d], static_cast<T>(n - 1))) : 0;  // NaN -> 0
+    f[d] = (c >= T(0)) ? static_cast<int>(fmin(c, static_cast<T>(n - 1))) : 0;  // NaN -> 0
   }
   const int bx = f[0] / PP_BRICK_X, by = f[1] / PP_BRICK_Y, bz = f[2] / PP_BRICK_Z;
   const int local = ((f[0] - bx * PP_BRICK_X) * PP_BRICK_Y + (f[1] - by * PP_BRICK_Y)) * PP_BRICK_Z +
@@ -256,33 +265,40 @@ __device__ __forceinline__ int brick_key(const BrickKeyArgs& b, unsigned s, T (&
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) brick_count(const BrickKeyArgs b, int32_t* count) {
+__global__ void __launch_bounds__(256) brick_count(const BrickKeyArgs b, int32_t* count, int32_t* keys) {
   const unsigned s = blockIdx.x * 256u + threadIdx.x;
   if (s >= static_cast<unsigned>(b.k.nvox)) return;
-  T c[3];
-  atomicAdd(count + brick_key<T>(b, s, c), 1);
+  const int key = brick_key<T>(b, s);
+  keys[s] = key;
+  atomicAdd(count + key, 1);
 }
 
 // The scatter pass: the scanned counts are cursors, advanced to their keys'
-// ends.  Each sample's key is formed again from the grid (12 bytes read; its
-// stored key and rank would be 8 bytes written and 8 read; the workspace still
-// has room for them, as its callers may have sized it).
-// Count and scatter of 192^3 samples, rough deformation: 42 + 125 us (65 + 117
-// with stored keys and ranks); 181 x 217 x 181, smoother: 42 + 83 us (59 + 76).  Bound by
-// scattered 4- and 16-byte writes; four samples per thread, for more atomics
-// in flight, spread the writes further: 154 us.  With `rec`, the
+// ends.  The keys are those that were counted, not formed again from the grid:
+// a grid that another stream writes meanwhile would send samples past the end
+// of `perm`.  Ranks need no storage (the workspace still has room for them, as
+// its callers may have sized it).
+// The order of 192^3 samples, rough deformation: 204 us (212 with ranks stored
+// too, 197 with keys formed twice); 160^3, smooth: 89 us (95, 85).  Bound by
+// scattered 4- and 16-byte writes; four samples per thread, for more atomics in
+// flight, spread the writes further (this pass 125 -> 154 us).  With `rec`, the
 // sample's coordinates and index also go as one 16-byte record to its place,
 // so that the brick kernels read each sample's data in brick order without
 // the perm -> grid indirection.
 template <class T>
-__global__ void __launch_bounds__(256) brick_scatter(const BrickKeyArgs b, int32_t* cursor, int32_t* perm, float4* rec) {
+__global__ void __launch_bounds__(256) brick_scatter(const BrickKeyArgs b, const int32_t* keys, int32_t* cursor,
+                                                     int32_t* perm, float4* rec) {
   const unsigned s = blockIdx.x * 256u + threadIdx.x;
   if (s >= static_cast<unsigned>(b.k.nvox)) return;
-  T c[3];
-  const int32_t pos = atomicAdd(cursor + brick_key<T>(b, s, c), 1);
+  const int32_t pos = atomicAdd(cursor + keys[s], 1);
   perm[pos] = static_cast<int32_t>(s);
-  if constexpr (sizeof(T) == 4)
-    if (rec) rec[pos] = make_float4(c[0], c[1], c[2], __int_as_float(static_cast<int>(s)));
+  if constexpr (sizeof(T) == 4) {
+    if (rec) {
+      unsigned v;
+      const T* g = sample_ptr<T>(b, s, v);
+      rec[pos] = make_float4(g[0], g[b.k.gsD], g[2 * b.k.gsD], __int_as_float(static_cast<int>(s)));
+    }
+  }
 }
 
 // brick_start[b] = end of the key before brick b's first; brick_start[nb] = nvox
@@ -338,6 +354,7 @@ int pp_brick_order(const pp_tensor* grid, const int64_t* src_size, int32_t* perm
   const int64_t nbricks = grid->sizes[0] * g.per_item;
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   int32_t* count = reinterpret_cast<int32_t*>(ws + L.count);
+  int32_t* keys = reinterpret_cast<int32_t*>(ws + L.keys);
   int32_t* partial = reinterpret_cast<int32_t*>(ws + L.partial);
   if ((rc = ppc::cuda_check(cudaMemsetAsync(count, 0, static_cast<size_t>(g.nkeys) * 4, st), "brick order clear")))
     return rc;
@@ -360,16 +377,16 @@ int pp_brick_order(const pp_tensor* grid, const int64_t* src_size, int32_t* perm
     b.nbx = static_cast<int>(g.nb[0]);
     b.nby = static_cast<int>(g.nb[1]);
     b.nbz = static_cast<int>(g.nb[2]);
-    if (grid->dtype == PP_FLOAT32) brick_count<float><<<nb, 256, 0, st>>>(b, count);
-    else brick_count<double><<<nb, 256, 0, st>>>(b, count);
+    if (grid->dtype == PP_FLOAT32) brick_count<float><<<nb, 256, 0, st>>>(b, count, keys);
+    else brick_count<double><<<nb, 256, 0, st>>>(b, count, keys);
     const int64_t ntile = (g.nkeys + SCAN_TILE - 1) / SCAN_TILE;
     scan_reduce<<<static_cast<unsigned>(ntile), SCAN_THREADS, 0, st>>>(count, g.nkeys, partial);
     scan_partials<<<1, SCAN_THREADS, 0, st>>>(partial, ntile);
     scan_apply<<<static_cast<unsigned>(ntile), SCAN_THREADS, 0, st>>>(count, g.nkeys, partial);
     if (grid->dtype == PP_FLOAT32)
-      brick_scatter<float><<<nb, 256, 0, st>>>(b, count, perm, reinterpret_cast<float4*>(records));
+      brick_scatter<float><<<nb, 256, 0, st>>>(b, keys, count, perm, reinterpret_cast<float4*>(records));
     else
-      brick_scatter<double><<<nb, 256, 0, st>>>(b, count, perm, nullptr);
+      brick_scatter<double><<<nb, 256, 0, st>>>(b, keys, count, perm, nullptr);
     ppc::count_launch(5);
   }
   brick_starts<<<static_cast<unsigned>((nbricks + 1 + 255) / 256), 256, 0, st>>>(count, nbricks,
