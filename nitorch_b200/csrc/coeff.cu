@@ -17,6 +17,7 @@
 // double with per-pole constants computed on the host.  Lines too long for a
 // shared tile fall back to the same recursion directly on global memory.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <type_traits>
 
@@ -666,22 +667,33 @@ int copy_any(const pp_tensor* in, const pp_tensor* out, cudaStream_t st) {
   }
 }
 
-template <class K>
-int allow_smem(K k, size_t smem, size_t static_bytes) {
-  // the 48 KB default covers static (line bases) plus dynamic shared memory
-  if (smem + static_bytes <= 48 * 1024) return PP_OK;
-  return ppc::cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                         "prefilter smem attribute");
+// Opts kernel K into `most` bytes of dynamic shared memory, the most that any
+// of its launches takes, once per device (bit d of `done`).  Set to each
+// launch's own size, the limit could drop below another thread's launch
+// between that thread's setting and its launch.
+template <auto K>
+int allow_smem(size_t most) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  if (int rc = ppc::cuda_check(cudaGetDevice(&dev), "prefilter device")) return rc;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load() & bit) return PP_OK;
+  if (int rc = ppc::cuda_check(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)),
+                               "prefilter smem attribute"))
+    return rc;
+  done.fetch_or(bit);
+  return PP_OK;
 }
+
+constexpr size_t TILE_SMEM = 113 * 1024, LONG_SMEM = 200 * 1024;  // two tiles per SM, one set of long lines
 
 template <class S, int NT, bool LM>
 int launch_tile(const LineArgs& a, cudaStream_t st) {
   using C = typename ppk::Acc<S>::type;
-  auto k = coeff_tile_kernel<S, NT, LM>;
   const size_t smem = static_cast<size_t>(a.n) * tile_pitch<C>(NT, LM) * sizeof(C);
-  if (int rc = allow_smem(k, smem, 2 * NT * sizeof(int64_t))) return rc;
+  if (int rc = allow_smem<coeff_tile_kernel<S, NT, LM>>(TILE_SMEM)) return rc;
   const int64_t blocks = (a.nlines + NT - 1) / NT;
-  k<<<static_cast<unsigned>(blocks), TILE_THREADS, smem, st>>>(a);
+  coeff_tile_kernel<S, NT, LM><<<static_cast<unsigned>(blocks), TILE_THREADS, smem, st>>>(a);
   ppc::count_launch();
   return ppc::cuda_check(cudaGetLastError(), "prefilter launch");
 }
@@ -715,14 +727,13 @@ int run_axis(LineArgs& a, cudaStream_t st) {
   using C = typename ppk::Acc<S>::type;
   constexpr int G = 16 / static_cast<int>(sizeof(C));
   if (a.nlines == 0) return PP_OK;
-  const size_t budget = 200 * 1024;
   // Full tiles: the widest NT (multiple of 32) whose tile leaves room for two
   // CTAs per SM, at most 64 lines where a line has four segments or more (all
   // threads recurse; at 96 lines there is room for two segments: 134 against
   // 92 us on 3 x 256^3, at 32 for eight: 117 us) and 128 where it has fewer
   // (4 x 400 x 400 lines of 40: 137 us at 64 lines, 94 at 128).
   {
-    const int64_t fit = static_cast<int64_t>(113 * 1024 / (static_cast<size_t>(a.n) * sizeof(C))) - 4;
+    const int64_t fit = static_cast<int64_t>(TILE_SMEM / (static_cast<size_t>(a.n) * sizeof(C))) - 4;
     // segments, each longer than a warm-up; with fewer than four their warm-ups
     // and checks cost what they save (cubic 72^3: 20.3 us in two, 19.0 whole)
     int64_t most = sizeof(C) == 4 ? a.n / (a.warm + 1) : 1;
@@ -737,7 +748,7 @@ int run_axis(LineArgs& a, cudaStream_t st) {
     }
   }
   // longer lines: fewer per CTA, one per thread
-  const int64_t fit = static_cast<int64_t>(budget / (static_cast<size_t>(a.n) * sizeof(C)));
+  const int64_t fit = static_cast<int64_t>(LONG_SMEM / (static_cast<size_t>(a.n) * sizeof(C)));
   int lines = static_cast<int>(fit < LL ? fit : LL), pitch = 0;
   if (a.line_major) {
     pitch = lines | 1;
@@ -748,15 +759,14 @@ int run_axis(LineArgs& a, cudaStream_t st) {
   }
   if (lines >= 1) {
     const size_t smem = static_cast<size_t>(a.n) * pitch * sizeof(C);
-    auto k = coeff_smem_kernel<S>;
-    if (int rc = allow_smem(k, smem, 2 * LL * sizeof(int64_t))) return rc;
+    if (int rc = allow_smem<coeff_smem_kernel<S>>(LONG_SMEM)) return rc;
     const int64_t blocks = (a.nlines + lines - 1) / lines;
-    k<<<static_cast<unsigned>(blocks), LL, smem, st>>>(a, pitch, lines);
+    coeff_smem_kernel<S><<<static_cast<unsigned>(blocks), LL, smem, st>>>(a, pitch, lines);
     ppc::count_launch();
   } else {
     if constexpr (sizeof(S) < 4) {
       return ppc::fail(PP_ERR_UNSUPPORTED, "(): 16-bit spline_coeff lines longer than %lld elements",
-                       (long long)(budget / sizeof(C)));
+                       (long long)(LONG_SMEM / sizeof(C)));
     } else {
       const int64_t blocks = (a.nlines + 127) / 128;
       coeff_global_kernel<S><<<static_cast<unsigned>(blocks), 128, 0, st>>>(a);
