@@ -254,11 +254,12 @@ def resize(image, factor=None, shape=None, affine=None, anchor="c", dim=None, *a
         out = resize_pull(x, scales, shifts, outshape, interpolation, bound, extrapolate)
     else:
         gdt = torch.float64 if x.dtype == torch.float64 else torch.float32
-        mat = torch.zeros((nb_dim, nb_dim + 1), dtype=gdt)
+        # filled by kernels: a copy from the host would wait for the GPU
+        mat = torch.zeros((nb_dim, nb_dim + 1), dtype=gdt, device=x.device)
         for d in range(nb_dim):
-            mat[d, d] = scales[d]
-            mat[d, nb_dim] = shifts[d]
-        out = affine_pull(x, mat.to(x.device), outshape, interpolation, bound, extrapolate)
+            mat[d, d].fill_(scales[d])
+            mat[d, nb_dim].fill_(shifts[d])
+        out = affine_pull(x, mat, outshape, interpolation, bound, extrapolate)
     out = out.reshape(*batch, *outshape)
     if affine is not None:
         affine = torch.as_tensor(affine)
