@@ -140,17 +140,17 @@ void set_grid(const pp_tensor* t, int D, int64_t& sN, int64_t s[3], int64_t& sD)
 
 bool fits32(int64_t v) { return v < (int64_t(1) << 31) - 1; }
 
-// Whether the direct kernels (pp_direct.cuh) serve a call: 3-D linear, 3-D
-// quadratic without a brick order and 2-D linear to cubic stencils of float32 /
-// bfloat16 images, plain or fused modes.
-// Higher orders, 64-bit offsets, deterministic scatters, coordinates computed
+// Whether the direct kernels (pp_direct.cuh) serve a call: 3-D linear and
+// quadratic and 2-D linear to cubic stencils of float32 / bfloat16 images,
+// plain or fused modes, in the grid's own order.
+// Calls with a sample order, higher orders, 64-bit offsets, deterministic scatters, coordinates computed
 // in the kernel and the interleaved accumulators keep their kernels.  Offsets
 // inside a batch item are 32-bit there (those of channels 64-bit, but for the
 // target's), so the element extent of every tensor must fit; batch items times
 // planes stay below 2^24 (the kernel divides them in float).
 bool direct_ok(int dtype, int D, int mode, int ord, bool wide, const ppk::PPArgs& a) {
-  if (wide || (dtype != PP_FLOAT32 && dtype != PP_BFLOAT16) || mode > ppk::K_PUSHGRAD) return false;
-  if (!(D == 3 && (ord == 1 || (ord == 2 && !a.brick_start))) && !(D == 2 && ord >= 1 && ord <= 3)) return false;
+  if (wide || a.perm || (dtype != PP_FLOAT32 && dtype != PP_BFLOAT16) || mode > ppk::K_PUSHGRAD) return false;
+  if (!(D == 3 && (ord == 1 || ord == 2)) && !(D == 2 && ord >= 1 && ord <= 3)) return false;
   if (a.det_acc || (a.flags & (ppk::F_VEC | ppk::F_IDGRID | ppk::F_ADDSELF | ppk::F_AFFINE)) || !ppk::lanes_enabled())
     return false;
   int64_t grid = (D - 1) * a.grid_sD, gg = (D - 1) * a.gg_sD, trgt = (a.C - 1) * a.trgt_sC;

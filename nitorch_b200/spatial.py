@@ -59,8 +59,8 @@ def set_sample_order(mode="auto"):
     """Processing order of the sampling points: "natural" (grid order),
     "sorted" (brick-major for 3-D grids, see pp_brick_order; source-sorted
     for 1-D / 2-D, see pp_sample_order) or "auto" (sorted for grids of at
-    least 2^18 points, but for calls of the direct kernels).  Only the speed
-    depends on it."""
+    least 2^18 points, but for the calls that the direct kernels take in grid
+    order, see _direct).  Only the speed depends on it."""
     global _sample_order_mode
     if mode not in ("auto", "natural", "sorted"):
         raise ValueError(f"unknown sample order mode {mode}")
@@ -161,25 +161,51 @@ def _brick_keys_fit(grid, src_size):
 _BRICK = (4, 4, 6)  # PP_BRICK_X, PP_BRICK_Y, PP_BRICK_Z
 
 
-def _direct(grid, interpolation, image):
+_INT = (1 << 31) - 1
+_direct_enabled = not os.environ.get("PP_PUSH_LANES", "").startswith("0")
+
+
+def _extent_fits(t):
+    """The element offsets inside a batch item fit 32 bits."""
+    if t.is_contiguous() and t.numel() < _INT:
+        return True
+    return sum((n - 1) * s for n, s in zip(t.shape[1:], t.stride()[1:])) < _INT
+
+
+def _direct(grid, src_size, interpolation, images):
     """The call runs the direct kernels (3-D linear and, for one channel,
     quadratic; 2-D linear to cubic; float32 / bfloat16 images), which take the
-    points in the grid's own order: no sort to pay for.  Quadratic on 160^3,
-    smooth and rough deformations: one channel 522-612 us in the grid's order
-    against 648-655 us sorted (forward + backward), two channels 920-1193
-    against 765-822.  `image`: (dtype, channels), or None for a call that the
-    direct kernels do not serve."""
-    if image is None or _deterministic or grid.dtype != torch.float32:
+    points in the grid's own order: no sort to pay for.  `images`: the call's
+    image tensors, or None for a call that the direct kernels do not serve.
+    The limits on sizes are pp_capi.cu's direct_ok: what it refuses runs the
+    kernels that gain from an order.  Both sides on 160^3 points of a new grid,
+    one call, us, in the grid's order against the per-point kernels with their
+    sort: displacements rough to white noise, linear pull 58 / 216 (3 channels
+    147 / 295), pull backward 159 / 361 (368 / 472); quadratic on smooth and
+    rough ones, forward + backward, one channel 522-612 / 648-655, two channels
+    920-1193 / 765-822.  Where neighbouring points lie far apart (axes
+    swapped), 1 channel still gains (linear pull 135 / 232, pull backward
+    271 / 380); more channels or taps do not (3 channels 408 / 323, quadratic
+    466 / 304), and "sorted" is faster for them."""
+    if images is None or _deterministic or not _direct_enabled or grid.dtype != torch.float32:
         return False
-    dtype, channels = image
+    dtype, channels = (images[0].dtype, images[0].shape[1]) if images else (grid.dtype, 1)
     dim = grid.dim() - 2
     order = int(interpolation[0])
     if dtype not in (torch.float32, torch.bfloat16) or any(int(i) != order for i in interpolation[1:dim]):
         return False
-    return order in (1, 2, 3) if dim == 2 else dim == 3 and (order == 1 or order == 2 and channels == 1)
+    if not (order in (1, 2, 3) if dim == 2 else dim == 3 and (order == 1 or order == 2 and channels == 1)):
+        return False
+    planes = grid.shape[0] * (grid.shape[1] if dim == 3 else 1)
+    source = 1
+    for n in src_size:
+        source *= int(n)
+    return (planes < (1 << 24) and grid.shape[dim - 1] <= 65535 and grid.numel() // grid.shape[0] < _INT
+            and grid.numel() // dim < _INT and source < _INT and _extent_fits(grid)
+            and all(_extent_fits(t) for t in images))
 
 
-def _order_for(grid, src_size, interpolation, image):
+def _order_for(grid, src_size, interpolation, images):
     """(perm, brick_start, records) for the call, or Nones for the natural
     order.  3-D grids get the brick-major order (it also drives the brick
     kernels); 1-D / 2-D grids the source-sorted one."""
@@ -187,7 +213,7 @@ def _order_for(grid, src_size, interpolation, image):
     if mode == "natural":
         return None, None, None
     nvox = grid.numel() // grid.shape[-1]
-    if mode == "auto" and (nvox < _SORT_MIN_SAMPLES or _direct(grid, interpolation, image)):
+    if mode == "auto" and (nvox < _SORT_MIN_SAMPLES or _direct(grid, src_size, interpolation, images)):
         return None, None, None
     if nvox >= (1 << 31):
         return None, None, None
@@ -287,9 +313,9 @@ def _grid32(grid):
     return grid
 
 
-def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, image=None):
+def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, images=None):
     _check_opts(bound, interpolation)
-    perm, starts, recs = (_order_for(grid, src_size, interpolation, image) if grid is not None and grid.is_cuda
+    perm, starts, recs = (_order_for(grid, src_size, interpolation, images) if grid is not None and grid.is_cuda
                           else (None, None, None))
     o = _lib.options([int(b) for b in bound], [int(i) for i in interpolation],
                      int(extrapolate), _lib.PP_DETERMINISTIC if _deterministic else 0,
@@ -326,7 +352,7 @@ def grid_pull(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]),
                       dtype=input.dtype, device=input.device)
     with _On(input):
@@ -342,7 +368,7 @@ def grid_pull_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input, grad))
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     ws, nws = _workspace(gi) if gi is not None else (None, 0)
@@ -384,7 +410,7 @@ def grid_push(input, grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, input.shape[2:], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape, (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, shape, (input,))
     out = torch.empty((grid.shape[0], input.shape[1], *shape), dtype=input.dtype, device=input.device)
     ws, nws = _workspace(out)
     with _On(input):
@@ -400,7 +426,7 @@ def grid_push_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (grad, input))
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     with _On(input):
@@ -428,7 +454,7 @@ def grid_count(grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, grid.shape[1:-1], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape, (g.dtype, 1))
+    opt = _opts(bound, interpolation, extrapolate, g, shape, ())
     out = torch.empty((grid.shape[0], 1, *shape), dtype=g.dtype, device=grid.device)
     ws, nws = _workspace(out)
     with _On(grid):
@@ -443,9 +469,9 @@ def grid_count_backward(grad, grid, bound, interpolation, extrapolate):
     _require_cuda(grid)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (g.dtype, 1))
-    gg = torch.empty(g.shape, dtype=g.dtype, device=g.device)
     gr = grad.to(g.dtype)
+    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (gr,))
+    gg = torch.empty(g.shape, dtype=g.dtype, device=g.device)
     with _On(grid):
         _lib.check(L.pp_grid_count_backward(ctypes.byref(_lib.desc(gr)), ctypes.byref(_lib.desc(g)),
                                             ctypes.byref(_lib.desc(gg)), ctypes.byref(opt),
@@ -463,7 +489,7 @@ def grid_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1], dim),
                       dtype=input.dtype, device=input.device)
@@ -483,7 +509,7 @@ def grid_pull_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input.dtype, input.shape[1]))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]), dtype=input.dtype,
                       device=input.device)
