@@ -121,9 +121,11 @@ PP_API const char* pp_last_error(void);
  * threads and devices); for auditing what ran on the GPU. */
 PP_API unsigned long long pp_kernel_launches(void);
 
-/* Kernel family, mode, order and channel block of the last push/pull
- * launch made on this host thread, e.g. "pp_brick_pullbwd_kernel mode=5 order=3
- * cb=3" ("" if none); for auditing which code path a call took. */
+/* Kernel family, mode, order and channel block of the last push / pull,
+ * resize, composition or regulariser launch made on this host thread, e.g.
+ * "pp_brick_pullbwd_kernel mode=5 order=3 cb=3" ("" if none); for auditing
+ * which code path a call took.  The resize family "resize_sep_kernel" names
+ * its form after it: "march" and / or "tma". */
 PP_API const char* pp_last_kernel(void);
 
 /* Workspace (device bytes, 256-byte aligned) that a push-type call with

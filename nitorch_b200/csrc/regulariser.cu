@@ -491,9 +491,23 @@ void launch_march(const RegArgs& A, int64_t N, cudaStream_t st) {
 
 // The marching kernel takes unweighted 3-D float32 grids whose neighbour
 // offsets fit 32 bits, in at most 65535 tiles along y and columns along x
-// and the batch; the others keep the kernel above.
-bool march_ok(const RegArgs& A, int64_t N) {
-  return A.narrow && (A.size[1] + RG_TY - 1) / RG_TY <= 65535 && N * ((A.size[0] + 7) / 8) <= 65535;
+// and the batch, where it is the faster one; the others keep the kernel above.
+// A column is 32 voxels wide along z and 8 along y whatever the volume has
+// there, and walks its planes one after another.  192 x 192 x Z, us, one
+// thread per voxel / marching: every term, Z = 4 20.9 / 26.4, 5 27.4 / 26.4,
+// 8 38 / 26; bending Z = 6 24.3 / 25.5, 8 31 / 25; Lame Z = 6 16.4 / 16.4;
+// radius 1 without it Z = 8 13.1 / 14.9, 10 15.4 / 14.9, 16 23 / 15.  Small
+// volumes, whose columns are few: radius 1 32^3 4.9 / 5.9 and 40^3 5.7 / 6.4,
+// with Lame 24^3 6.9 / 7.0, bending 16^3 9.1 / 9.8 and 20^3 9.8 / 9.5 (a plane
+// or two take no walk: radius 1 1 x 96^2 4.4 / 4.1).
+bool march_ok(const RegArgs& A, int64_t N, int R, bool lame) {
+  if (!A.narrow || (A.size[1] + RG_TY - 1) / RG_TY > 65535 || N * ((A.size[0] + 7) / 8) > 65535) return false;
+  const double across = static_cast<double>(A.size[1]) * A.size[2];
+  const double covered = static_cast<double>((A.size[1] + RG_TY - 1) / RG_TY * RG_TY) *
+                         ((A.size[2] + RG_TZ - 1) / RG_TZ * RG_TZ);
+  const double most = R == 1 && !lame ? 3.2 : R == 2 && lame ? 6.4 : R == 2 ? 5.0 : 4.0;
+  const int64_t least = R == 2 ? 6000 : lame ? 1 << 15 : 1 << 17;
+  return covered <= most * across && (A.nvox >= least || A.size[0] <= 2);
 }
 
 // ---- host ------------------------------------------------------------------
@@ -555,7 +569,9 @@ bool narrow_ok(const pp_tensor* t) { return !t || 4 * ppc::max_offset(t, 1) < (i
 int launch(RegArgs& A, int dtype, int dim, bool grid, int R, bool W, bool lame, cudaStream_t st) {
   if (A.nvox == 0) return PP_OK;
   const int64_t N = A.nvox / (int64_t(A.size[0]) * A.size[1] * A.size[2]);
-  if (dtype == PP_FLOAT32 && dim == 3 && grid && !W && march_ok(A, N)) {
+  const bool march = dtype == PP_FLOAT32 && dim == 3 && grid && !W && march_ok(A, N, R, lame);
+  ppk::note_kernel(march ? "regulariser_march_kernel" : "regulariser_kernel", 0, R, A.C);
+  if (march) {
     if (R == 2) lame ? launch_march<2, true>(A, N, st) : launch_march<2, false>(A, N, st);
     else lame ? launch_march<1, true>(A, N, st) : launch_march<1, false>(A, N, st);
   } else if (dtype == PP_FLOAT32) {
