@@ -75,6 +75,7 @@ struct BrickArgs {
   PPArgs p;
   float lo, hi[3];
   int per_item;             // samples of a batch item
+  int chunk, nchunk;        // samples per chunk, chunks (see brick_chunk)
   int lin;                  // out_l, trgt_l, gg_l hold
   int out_l, trgt_l, gg_l;  // elements per sample
 };
@@ -190,6 +191,57 @@ __device__ __forceinline__ BrickPos brick_pos(const PPArgs& a, int b) {
   q.interior = q.ox >= 0 && q.oy >= 0 && q.oz >= 0 && q.ox + W::EX <= a.src_size[0] &&
                q.oy + W::EY <= a.src_size[1] && q.oz + W::EZ <= a.src_size[2];
   return q;
+}
+
+// Dense bricks.  One CTA or warp for a brick of far more samples than its
+// share (a grid that samples few voxels of its source, a small source, points
+// outside the volume collected in its edge bricks) would outlast the others by
+// far.  So the samples in brick order are also cut into chunks of b.chunk, and
+// bricks (scatter) or columns of a group's bricks (gathers) of that many
+// samples or more are left to one CTA or warp per chunk: the last b.nchunk of
+// the launch, of which those whose chunk does not begin in a dense brick have
+// nothing to do.  (At the launch's start they delay the others, and leave the
+// groups of small sources unevenly on the SMs: 64^3, 66 -> 90 us.)  A chunk's work ends where the next begins or its bricks end,
+// and starts with their first sample where no chunk begins before it.
+// Chunks are longer than what bricks hold of grids up to twice as dense as
+// their source, whose windows are then staged or added once.
+// 160^3 samples of one channel, cubic, without chunks / with them: of 20^3
+// voxels, pull 1020 / 68 us, push 2990 / 188, pull backward 4540 / 280, spatial
+// gradient 1380 / 89 (per point 250); of twice the volume, mirrored at its
+// edges, gradient 49.6 / 0.94 ms (per point 0.66); dense grids as without.
+__device__ __forceinline__ float4 brick_sample(const PPArgs& a, int p);
+
+// Brick that holds the sample at position p of the brick order: the one that
+// its coordinates name, or by bisection (a grid written since it was ordered).
+__device__ __forceinline__ int brick_of(const BrickArgs& b, int p) {
+  const PPArgs& a = b.p;
+  const float4 r = brick_sample(a, p);
+  const float x[3] = {r.x, r.y, r.z};
+  const int nbricks = static_cast<int>(a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2]);
+  int q = __float_as_int(r.w) / b.per_item;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int f = x[d] >= 0.f ? static_cast<int>(fminf(x[d], static_cast<float>(a.src_size[d] - 1))) : 0;
+    q = q * static_cast<int>(a.nbrick[d]) + f / (d == 0 ? BRK_X : d == 1 ? BRK_Y : BRK_Z);
+  }
+  q = min(max(q, 0), nbricks - 1);
+  if (__ldg(a.brick_start + q) <= p && p < __ldg(a.brick_start + q + 1)) return q;
+  int lo = 0, hi = nbricks;  // brick_start[lo] <= p < brick_start[hi]
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (__ldg(a.brick_start + m) <= p) lo = m;
+    else hi = m;
+  }
+  return lo;
+}
+
+// Samples [s0, s1) that chunk c is to work on, of those [s0, s1) of the bricks
+// that its first sample lies in: empty if they are not dense.
+__device__ __forceinline__ void brick_chunk(const BrickArgs& b, int c, int& s0, int& s1) {
+  const int p = c * b.chunk;
+  const bool dense = s1 - s0 >= b.chunk;
+  if (p - b.chunk >= s0) s0 = p;
+  s1 = dense ? (s1 - p > b.chunk ? p + b.chunk : s1) : s0;
 }
 
 // Window voxel e (x slowest, z fastest) -> window coordinates.
@@ -419,10 +471,13 @@ __global__ void __launch_bounds__(32 * BRK_SCATTER_WARPS, 6) pp_brick_scatter_ke
   float* acc = reinterpret_cast<float*>(brick_smem4) + wid * SM::PER_WARP;
   float* rec = acc + W::NV * CP;
 
-  const int nbricks = static_cast<int>(a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2]);
-  const int brick = static_cast<int>(blockIdx.x) * BRK_SCATTER_WARPS + wid;
-  if (brick >= nbricks) return;  // whole warp
-  const int p0 = __ldg(a.brick_start + brick), p1 = __ldg(a.brick_start + brick + 1);
+  int brick = static_cast<int>(blockIdx.x) * BRK_SCATTER_WARPS + wid;
+  const int chunk = brick - static_cast<int>(a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2]);
+  if (chunk >= b.nchunk) return;  // whole warp
+  if (chunk >= 0) brick = brick_of(b, chunk * b.chunk);
+  int p0 = __ldg(a.brick_start + brick), p1 = __ldg(a.brick_start + brick + 1);
+  if (chunk >= 0) brick_chunk(b, chunk, p0, p1);
+  else if (p1 - p0 >= b.chunk) return;  // its chunks' work
   if (p0 >= p1) return;
   const BrickPos bp = brick_pos(a, brick);
 
@@ -521,21 +576,38 @@ __device__ __forceinline__ void brick_gather(const BrickArgs& b) {
   const PPArgs& a = b.p;
   const int nx = static_cast<int>(a.nbrick[0]), ny = static_cast<int>(a.nbrick[1]), nz = static_cast<int>(a.nbrick[2]);
   const int gx = (nx + GRP - 1) / GRP, gy = (ny + GRP - 1) / GRP, gz = (nz + GRP - 1) / GRP;
-  int r = static_cast<int>(blockIdx.x);
-  const int bz = r % gz * GRP; r /= gz;
-  const int by = r % gy * GRP; r /= gy;
-  const int bx = r % gx * GRP;
-  const int n = r / gx;
-  if (threadIdx.x < 4) {
-    const int x = bx + static_cast<int>(threadIdx.x >> 1), y = by + static_cast<int>(threadIdx.x & 1);
-    int s0 = 0, cnt = 0;
-    if (x < nx && y < ny) {
+  const int chunk = static_cast<int>(blockIdx.x) - static_cast<int>(a.N) * gx * gy * gz;
+  int bx, by, bz, n, s0 = 0, s1 = 0;  // s0, s1: a chunk's samples, or those of a column (threads 0 - 3)
+  if (chunk >= 0) {
+    int r = brick_of(b, chunk * b.chunk);
+    bz = r % nz & -GRP;
+    const int q = r - r % nz + bz;
+    s0 = __ldg(a.brick_start + q);
+    s1 = __ldg(a.brick_start + q + min(GRP, nz - bz));
+    brick_chunk(b, chunk, s0, s1);
+    if (s0 >= s1) return;  // whole CTA
+    if (threadIdx.x) s0 = s1 = 0;
+    r /= nz;
+    by = r % ny; r /= ny;
+    bx = r % nx;
+    n = r / nx;
+  } else {
+    int r = static_cast<int>(blockIdx.x);
+    bz = r % gz * GRP; r /= gz;
+    by = r % gy * GRP; r /= gy;
+    bx = r % gx * GRP;
+    n = r / gx;
+    const int x = bx + static_cast<int>(threadIdx.x >> 1 & 1u), y = by + static_cast<int>(threadIdx.x & 1);
+    if (threadIdx.x < 4 && x < nx && y < ny) {
       const int q = ((n * nx + x) * ny + y) * nz + bz;
       s0 = __ldg(a.brick_start + q);
-      cnt = __ldg(a.brick_start + q + min(GRP, nz - bz)) - s0;
+      s1 = __ldg(a.brick_start + q + min(GRP, nz - bz));
+      if (s1 - s0 >= b.chunk) s1 = s0;  // its chunks' work
     }
+  }
+  if (threadIdx.x < 4) {
     first[threadIdx.x] = s0;
-    int inc = cnt;
+    int inc = s1 - s0;
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {
       const int u = __shfl_up_sync(0xfu, inc, o);
@@ -543,6 +615,8 @@ __device__ __forceinline__ void brick_gather(const BrickArgs& b) {
     }
     upto[threadIdx.x] = inc;
   }
+  bx &= -GRP;
+  by &= -GRP;
   const int ox = bx * BRK_X - 1, oy = by * BRK_Y - 1, oz = bz * BRK_Z - 1;
   if (threadIdx.x >= 32 && threadIdx.x < 32 + 48) {
     static_assert(G::EX <= 16 && G::EY <= 16 && G::EZ <= 16, "window tables");
@@ -741,29 +815,39 @@ __global__ void __launch_bounds__(BRK_GATHER_THREADS, GatherBlocks<K_PUSHGRAD, C
 
 // Dynamic shared memory above 48 KB must be opted into, once per kernel and
 // device: `done` is the caller's per-instantiation record of the devices
-// already set up (bit d = device d).
+// already set up (bit d = device d).  `carve`: percentage of the unified L1 /
+// shared array that the resident CTAs' windows need.
 template <class K>
-inline cudaError_t brick_smem_optin(K kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+inline cudaError_t brick_smem_optin(K kernel, size_t bytes, std::atomic<unsigned long long>& done,
+                                    int carve = cudaSharedmemCarveoutMaxShared) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  // the whole unified L1 / shared array as shared memory: several CTAs of
-  // these window-sized allocations per SM
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
   if (e == cudaSuccess) done.fetch_or(bit);
   return e;
 }
 
+// Chunks of a power of two samples, `least` or more, up to `most` chunks.
+inline void set_chunks(BrickArgs& b, int64_t most, int64_t least) {
+  int64_t chunk = least;
+  while (chunk * most < b.p.nvox) chunk *= 2;
+  b.chunk = static_cast<int>(chunk);
+  b.nchunk = static_cast<int>((b.p.nvox + chunk - 1) / chunk);
+}
+
 template <int MODE, int ORD, int CB, class S>
-inline cudaError_t launch_brick_scatter(const BrickArgs& b, cudaStream_t st) {
+inline cudaError_t launch_brick_scatter(BrickArgs b, cudaStream_t st) {
   constexpr int CP = CB;  // 3: channel planes
   constexpr size_t bytes = BrickScatterSmem<CP>::bytes;
   const PPArgs& a = b.p;
-  const int64_t grid = (a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2] + BRK_SCATTER_WARPS - 1) / BRK_SCATTER_WARPS;
+  set_chunks(b, 148 * 6 * BRK_SCATTER_WARPS, 1024);  // up to one per resident warp
+  const int64_t grid =
+      (b.nchunk + a.N * a.nbrick[0] * a.nbrick[1] * a.nbrick[2] + BRK_SCATTER_WARPS - 1) / BRK_SCATTER_WARPS;
   static std::atomic<unsigned long long> optin_done{0};  // one per kernel instantiation
   cudaError_t e = brick_smem_optin(pp_brick_scatter_kernel<MODE, ORD, CB, CP, S>, bytes, optin_done);
   if (e != cudaSuccess) return e;
@@ -773,20 +857,27 @@ inline cudaError_t launch_brick_scatter(const BrickArgs& b, cudaStream_t st) {
 }
 
 template <int MODE, int ORD, int CB, class S>
-inline cudaError_t launch_brick_gather(const BrickArgs& b, cudaStream_t st) {
+inline cudaError_t launch_brick_gather(BrickArgs b, cudaStream_t st) {
   constexpr int CP = CB == 3 ? 4 : CB;
   constexpr size_t bytes = BrickGatherSmem<CP>::bytes;
   const PPArgs& a = b.p;
+  set_chunks(b, 4 * 148 * GatherBlocks<MODE, CB>::value, 2048);  // up to four per resident CTA
   int64_t grid = a.N;
   for (int d = 0; d < 3; ++d) grid *= (a.nbrick[d] + GRP - 1) / GRP;
+  grid += b.nchunk;
   static std::atomic<unsigned long long> optin_done{0};
+  // the rest stays L1, for the samples' scattered reads and writes and the
+  // points past the window (160^3, one channel, all of it as shared memory: pull
+  // 143 -> 132 us, gradient 166 -> 152; mostly outside points 1.88 -> 1.14 ms)
+  constexpr int carve = static_cast<int>(
+      std::min<size_t>(100, (bytes + 3584) * GatherBlocks<MODE, CB>::value * 100 / (228 * 1024) + 1));
   if constexpr (MODE == K_PUSHGRAD) {
-    cudaError_t e = brick_smem_optin(pp_brick_pullbwd_kernel<ORD, CB, CP, S>, bytes, optin_done);
+    cudaError_t e = brick_smem_optin(pp_brick_pullbwd_kernel<ORD, CB, CP, S>, bytes, optin_done, carve);
     if (e != cudaSuccess) return e;
     note_kernel("pp_brick_pullbwd_kernel", MODE, ORD, CB);
     pp_brick_pullbwd_kernel<ORD, CB, CP, S><<<static_cast<unsigned>(grid), BRK_GATHER_THREADS, bytes, st>>>(b);
   } else {
-    cudaError_t e = brick_smem_optin(pp_brick_gather_kernel<MODE, ORD, CB, CP, S>, bytes, optin_done);
+    cudaError_t e = brick_smem_optin(pp_brick_gather_kernel<MODE, ORD, CB, CP, S>, bytes, optin_done, carve);
     if (e != cudaSuccess) return e;
     note_kernel("pp_brick_gather_kernel", MODE, ORD, CB);
     pp_brick_gather_kernel<MODE, ORD, CB, CP, S><<<static_cast<unsigned>(grid), BRK_GATHER_THREADS, bytes, st>>>(b);
