@@ -205,7 +205,23 @@ def _direct(grid, src_size, interpolation, images):
             and all(_extent_fits(t) for t in images))
 
 
-def _order_for(grid, src_size, interpolation, images):
+def _brick_least(op, interpolation):
+    """Samples from which the brick kernels are faster than one thread per point
+    over the same order, for the calls where that depends on it: a CTA's window
+    and the points past the volume's edges cost small volumes more.  Per point /
+    bricks, smooth displacements, us: cubic spatial gradient 64^3 24 / 28, 80^3
+    36 / 36, 96^3 65 / 47 (3 channels 48 / 57, 69 / 83, 134 / 100); push
+    backward 64^3 25 / 30, 80^3 37 / 40; quadratic pull 64^3 20 / 22, push 80^3
+    55 / 65, 96^3 85 / 80, pull backward 96^3 132 / 149."""
+    order = int(interpolation[0])
+    if op == "grad":
+        return 550_000
+    if order == 2:
+        return {"pull": 550_000, "push": 700_000, "pull_backward": 1_100_000}.get(op, 0)
+    return 0
+
+
+def _order_for(grid, src_size, interpolation, images, op=None):
     """(perm, brick_start, records) for the call, or Nones for the natural
     order.  3-D grids get the brick-major order (it also drives the brick
     kernels); 1-D / 2-D grids the source-sorted one."""
@@ -222,6 +238,8 @@ def _order_for(grid, src_size, interpolation, images):
     if entry is None:
         entry = brick_order(grid, src_size) if bricks else (sample_order(grid, src_size), None, None)
         _orders.put(grid, src_size, entry)
+    if mode == "auto" and bricks and nvox < _brick_least(op, interpolation):
+        return entry[0], None, None
     return entry
 
 
@@ -313,9 +331,9 @@ def _grid32(grid):
     return grid
 
 
-def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, images=None):
+def _opts(bound, interpolation, extrapolate, grid=None, src_size=None, images=None, op=None):
     _check_opts(bound, interpolation)
-    perm, starts, recs = (_order_for(grid, src_size, interpolation, images) if grid is not None and grid.is_cuda
+    perm, starts, recs = (_order_for(grid, src_size, interpolation, images, op) if grid is not None and grid.is_cuda
                           else (None, None, None))
     o = _lib.options([int(b) for b in bound], [int(i) for i in interpolation],
                      int(extrapolate), _lib.PP_DETERMINISTIC if _deterministic else 0,
@@ -352,7 +370,7 @@ def grid_pull(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,), "pull")
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]),
                       dtype=input.dtype, device=input.device)
     with _On(input):
@@ -368,7 +386,7 @@ def grid_pull_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input, grad))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input, grad), "pull_backward")
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     ws, nws = _workspace(gi) if gi is not None else (None, 0)
@@ -410,7 +428,7 @@ def grid_push(input, grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, input.shape[2:], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape, (input,))
+    opt = _opts(bound, interpolation, extrapolate, g, shape, (input,), "push")
     out = torch.empty((grid.shape[0], input.shape[1], *shape), dtype=input.dtype, device=input.device)
     ws, nws = _workspace(out)
     with _On(input):
@@ -426,7 +444,7 @@ def grid_push_backward(grad, input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (grad, input))
+    opt = _opts(bound, interpolation, extrapolate, g, grad.shape[2:], (grad, input), "grad")
     gi = torch.empty_like(input, memory_format=torch.contiguous_format) if input.requires_grad else None
     gg = torch.empty(g.shape, dtype=g.dtype, device=g.device) if grid.requires_grad else None
     with _On(input):
@@ -454,7 +472,7 @@ def grid_count(grid, shape, bound, interpolation, extrapolate):
     shape = _push_shape(shape, grid.shape[1:-1], dim)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, shape, ())
+    opt = _opts(bound, interpolation, extrapolate, g, shape, (), "push")
     out = torch.empty((grid.shape[0], 1, *shape), dtype=g.dtype, device=grid.device)
     ws, nws = _workspace(out)
     with _On(grid):
@@ -489,7 +507,7 @@ def grid_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,), "grad")
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1], dim),
                       dtype=input.dtype, device=input.device)
@@ -509,7 +527,7 @@ def grid_pull_grad(input, grid, bound, interpolation, extrapolate):
     _require_cuda(input)
     L = _lib.load()
     g = _grid32(grid)
-    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,))
+    opt = _opts(bound, interpolation, extrapolate, g, input.shape[2:], (input,), "grad")
     dim = grid.dim() - 2
     out = torch.empty((grid.shape[0], input.shape[1], *grid.shape[1:-1]), dtype=input.dtype,
                       device=input.device)

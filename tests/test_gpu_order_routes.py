@@ -56,3 +56,17 @@ def test_refused_sizes_keep_their_order(monkeypatch):
     assert len(orders) == 1 and not any(k.startswith("pp_direct_kernel") for k in kernels)
     for a, r in zip(out, ref):
         assert float((a - r).abs().max() / r.abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("n,order,bricks", [(66, 3, (True, False, True, True)), (66, 2, (False, False, False, False)),
+                                            (84, 3, (True, True, True, True)), (84, 2, (True, True, False, False))])
+def test_small_volumes_run_per_point(n, order, bricks):
+    """Ordered grids of 2^18 points and more whose windows do not pay."""
+    spatial.set_sample_order("natural")
+    ref, _ = _calls((n, n, n), (n, n, n), order)
+    spatial.set_sample_order("auto")
+    out, kernels = _calls((n, n, n), (n, n, n), order)
+    assert tuple(k.startswith("pp_brick_") for k in kernels) == bricks, kernels
+    assert not any(k.startswith("pp_direct_") for k in kernels), kernels
+    for a, r in zip(out, ref):
+        assert float((a - r).abs().max() / r.abs().max()) < 1e-5
