@@ -417,11 +417,12 @@ inline cudaError_t launch_direct(const PPArgs& p, cudaStream_t st) {
   a.outer = static_cast<int>(p.N) * a.X;
   a.invX = 1.f / static_cast<float>(a.X);
   a.C = static_cast<int>(p.C); a.extrapolate = p.extrapolate; a.flags = p.flags;
-  // the tile's extent along the last axis: 32, or 16 or 8 where that covers
-  // the grid with at least an eighth fewer threads
+  // the tile's extent along the last axis: 32, or what covers the grid with at
+  // least an eighth fewer threads (256 x 256 x 2, linear, in tiles of 8 / 2
+  // along z: push 13.4 / 6.7, pull backward 19.1 / 8.7 us)
   a.tzs = 5;
   int64_t best = 0;
-  for (int s = 5; s >= 3; --s) {
+  for (int s : {5, 4, 3, 2, 1, 0, 6, 7, 8}) {
     const int tz = 1 << s, ty = DIR_THREADS >> s;
     const int64_t cover = static_cast<int64_t>((a.Z + tz - 1) / tz * tz) * ((a.Y + ty - 1) / ty * ty);
     if (s == 5 || cover * 8 < best * 7) { best = cover; a.tzs = s; }
