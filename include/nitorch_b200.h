@@ -267,7 +267,7 @@ PP_API int pp_affine_grad_matrix(const pp_tensor* grad, const pp_tensor* input, 
  * 618-754, affine_grid then ni::grid_pull) and of its native ni::resize
  * (nitorch/_C/src/resize.h, resize_common.cpp:600-700, which extrapolates:
  * set bit 0 of opt->extrapolate).  Computed separably (three 4-tap passes
- * over TMA-staged tiles); equal to pp_affine_pull with the diagonal matrix.
+ * over TMA-staged tiles); pp_affine_pull with the diagonal matrix, to rounding.
  * Other cases return PP_ERR_UNSUPPORTED (use pp_affine_pull). */
 PP_API int pp_resize(const pp_tensor* input, const pp_tensor* out, const double* scale, const double* shift,
                      const pp_options* opt, void* stream);

@@ -250,7 +250,7 @@ def resize(image, factor=None, shape=None, affine=None, anchor="c", dim=None, *a
     if prefilter:
         x = spline_coeff_nd(x, interpolation=interpolation, bound=bound, dim=nb_dim)
     if nb_dim == 3 and all(s > 0 for s in scales) and resize_supported(x, interpolation):
-        # diagonal map: the separable kernel (equal to the affine pull)
+        # diagonal map: the separable kernels (the affine pull, to rounding)
         out = resize_pull(x, scales, shifts, outshape, interpolation, bound, extrapolate)
     else:
         gdt = torch.float64 if x.dtype == torch.float64 else torch.float32

@@ -1298,10 +1298,11 @@ inline cudaError_t launch_one(const PPArgs& a, cudaStream_t st) {
           return cudaGetLastError();
         }
       }
-      // linear pull backward with up to CB channels (the self-composition
-      // backward of velocity exponentiation included): lane-split with
-      // scalar reductions into the output.  (Cubic single-channel images
-      // measured slower this way: 1.43 -> 1.59 ms on a 192^3 grid.)
+      // linear pull backward with up to CB channels: lane-split with scalar
+      // reductions into the output.  Reached with a sample order, by sizes that
+      // the direct kernels refuse, and by self-compositions that svf_compose.cu
+      // does not take.  (Cubic single-channel images measured slower this way:
+      // 1.43 -> 1.59 ms on a 192^3 grid.)
       if constexpr (ORD == 1) {
         if (!(a.flags & F_VEC) && a.C <= CB) {
           note_kernel("pp_lanes_pullbwd_kernel", MODE, ORD, CB);

@@ -394,7 +394,8 @@ __global__ void __launch_bounds__(RG_THREADS, 2) regulariser_march_kernel(const 
     }
     __syncthreads();
     if (x + 1 < x1) fetch(x + R + 1);
-    // a plane is rewritten three iterations after its last reader's barrier
+    // plane x is last read here; plane x + 4 takes its slot 4 - R iterations on,
+    // behind the barriers between
     const float* p0 = slot(x) + me;
     const float* p1 = slot(x + 1) + me;
     const float* pr = slot(x + R) + me;

@@ -21,8 +21,9 @@
 //      y pass: T2[ox][oy][z] = sum_j wy_j T1[ox][ly + j][z];
 //      z pass: out = sum_k wz_k T2[ox][oy][lz + k], stored along z.
 // Each partial sum is the fused multiply-add chain of the per-point kernel
-// (x innermost, then y, then z, starting from zero), so the result equals
-// pp_grid_pull's on the materialised affine grid.  Persistent CTAs walk the
+// (x innermost, then y, then z, starting from zero), so these tiles' result equals
+// pp_grid_pull's on the materialised affine grid (the marching form further
+// down, for moderate steps, sums z, y, x: equal to rounding).  Persistent CTAs walk the
 // (tile, channel) items with two staging buffers: the next item's copy is
 // in flight while the current item is filtered; the x and y passes move
 // four z positions per thread (16-byte shared accesses).
