@@ -289,10 +289,10 @@ SCATTER_OPS = ("push_fwd", "pull_bwd", "pp_fwd", "pp_bwd")
 # channel-interleaved accumulator into the output (store_interleaved_vox).
 # A kernel not listed here reports traffic null.
 MEASURED_TRAFFIC = {
-    "pp_brick_gather_kernel mode=0 order=3 cb=3": 289_696_256,
-    "pp_brick_scatter_kernel mode=2 order=3 cb=3": 399_176_192 + 146_609_152,
-    "pp_brick_gather_kernel mode=4 order=3 cb=3": 523_536_384,
-    "pp_brick_pullbwd_kernel mode=5 order=3 cb=3": 400_533_504 + 379_292_416 + 146_874_368,
+    "pp_brick_gather_kernel mode=0 order=3 cb=3": 291_238_400,
+    "pp_brick_scatter_kernel mode=2 order=3 cb=3": 400_127_488 + 146_951_424,
+    "pp_brick_gather_kernel mode=4 order=3 cb=3": 523_825_408,
+    "pp_brick_pullbwd_kernel mode=5 order=3 cb=3": 399_324_160 + 377_071_616 + 147_655_936,
 }
 
 

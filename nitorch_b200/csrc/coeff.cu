@@ -359,10 +359,9 @@ struct alignas(4 * sizeof(S)) Quad {
 // filtered by a.nseg of them (filter_segment).  With one thread per line the
 // recursions, two dependent passes of n steps, took longer than the
 // transfers: at 64 lines per CTA and four segments of 64 samples (warm-ups of
-// 23) per line of 256, three CTAs per SM, a pass over 3 x 256^3 floats takes
-// 91 / 87 / 107 us (first / middle / last axis; 136 / 121 / 150 with one
-// thread per line and 96 lines per CTA), 62 us of it memory traffic at the
-// copy rate; 3 x 192^3 48 / 48 / 50 us (55 / 55 / 69).  More registers per
+// 23) per line of 256, three CTAs per SM, the three axes of 3 x 256^3 floats
+// take 280 us (374 with one thread per line and 96 lines per CTA), 187 us of it
+// memory traffic at the copy rate; 3 x 192^3 128 us (149).  More registers per
 // thread or a fourth CTA per SM gain nothing further.
 //  * filtered axis the fastest (LM): a warp instruction covers 8 groups of
 //    four consecutive samples of 4 lines (128-byte segments), through

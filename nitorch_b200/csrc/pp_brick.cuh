@@ -42,10 +42,10 @@
 //
 // Measured on 3 x 192^3, cubic, rough deformation (std 4 over 2 voxels), one
 // brick per CTA (push backward: the per-point kernel) before and this form
-// after: pull 0.654 -> 0.419 ms, push backward 1.111 -> 0.657 ms, pull
-// backward (was one kernel for both gradients) 1.755 -> 0.670 + 0.596 ms, push
-// 0.731 -> 0.596 ms.  160 x 192 x 160, one channel: pull 0.322 -> 0.171 ms,
-// grid gradient 0.583 -> 0.282 ms.  The gathers are latency-bound (scattered
+// after: pull 0.654 -> 0.405 ms, push backward 1.111 -> 0.555 ms, pull
+// backward (was one kernel for both gradients) 1.755 -> 0.572 + 0.603 ms, push
+// 0.731 -> 0.603 ms.  160 x 192 x 160, one channel: pull 0.322 -> 0.158 ms,
+// grid gradient 0.583 -> 0.236 ms.  The gathers are latency-bound (scattered
 // reads and writes by sample index, three or four CTAs per SM).
 //
 // Points whose support leaves the window (sampling outside the volume with
@@ -448,7 +448,7 @@ __device__ __forceinline__ void scatter_walk(float* acc, const float* rec, int c
 // Sums runs first where a warp's points have enough of them: at one run per
 // point the walk with runs takes up to 7 % longer (smooth deformations), at
 // 0.63 runs per point (independent uniform positions) 9 % less: 3 x 192^3,
-// rough, 0.652 -> 0.596 ms.  It also rounds less often.
+// rough, 0.652 -> 0.600 ms.  It also rounds less often.
 template <int ORD, int CP>
 __device__ __forceinline__ void scatter_recorded(float* acc, const float* rec, int cnt, int lane) {
   const int at = lane < cnt ? __float_as_int(rec[lane * BRK_REC + (CP < 4 ? 15 : 16)]) : -1;

@@ -28,7 +28,7 @@
 // (std 3 over 6 voxels), per-point / lane-split kernels before and these
 // after: pull 205 -> 120 us, pull backward 555 -> 311 us, and the 255 us
 // sort is gone; push of 256^3 627 -> 298 us; 4 x 8 x 512^2 cubic pull 178 ->
-// 75 us, backward 482 -> 213 us.  What bounds them: instruction issue (58 %
+// 75 us, backward 482 -> 218 us.  What bounds them: instruction issue (58 %
 // active, ~245 instructions per linear pull) and L1 latency for the gathers,
 // the reductions' sectors through L1 and L2 (72 % and 57 % of peak) for the
 // scatters.
@@ -118,7 +118,7 @@ template <int D, int ORD, int MODE, int CB> struct DirBlocks {
 // of all channels first, one sum over the nodes of their dot product; fewer
 // registers, but the differences then carry the rounding of the products (rms
 // error of 2-D linear gradients of a smooth 4-channel image: 4.7e-7 against
-// 2.2e-7; 4 x 8 x 512^2 cubic, both passes: 301 and 308 us).  Only the
+// 2.2e-7; 4 x 8 x 512^2 cubic, both passes: 293 and 300 us).  Only the
 // 3-D linear pull backward of two to four channels sums so, as its lane-split
 // kernel (pp_lanes_pullbwd_kernel) does.
 template <int D, int ORD, int CB, class S, int MODE, bool DOT>
