@@ -380,7 +380,7 @@ constexpr int TILE_THREADS = 256;
 
 template <class C> constexpr int tile_pitch(int nt, bool line_major) { return line_major && sizeof(C) == 4 ? nt + 1 : nt + 4; }
 
-template <class S, int NT, bool LM>
+template <class S, int NT, bool LM, bool SEG>
 __global__ void __launch_bounds__(TILE_THREADS, sizeof(S) == 8 ? 2 : 3) coeff_tile_kernel(LineArgs a) {
   using C = typename ppk::Acc<S>::type;
   constexpr int G = 16 / static_cast<int>(sizeof(C));
@@ -462,8 +462,8 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(S) == 8 ? 2 : 3) coeff_ti
   if constexpr (kAsync) asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   const int col = threadIdx.x % NT, seg = threadIdx.x / NT;
-  const bool active = seg < a.nseg && col < nl;
-  if (a.nseg > 1) {
+  const bool active = seg < (SEG ? a.nseg : 1) && col < nl;
+  if constexpr (SEG) {
     filter_segment(TileCol<C, P>{sm + col}, n32, a, seg, active);
   } else {
     if (active) filter_line(TileCol<C, P>{sm + col}, n32, a);
@@ -686,28 +686,35 @@ int allow_smem(size_t most) {
 
 constexpr size_t TILE_SMEM = 113 * 1024, LONG_SMEM = 200 * 1024;  // two tiles per SM, one set of long lines
 
-template <class S, int NT, bool LM>
+template <class S, int NT, bool LM, bool SEG>
 int launch_tile(const LineArgs& a, cudaStream_t st) {
   using C = typename ppk::Acc<S>::type;
   const size_t smem = static_cast<size_t>(a.n) * tile_pitch<C>(NT, LM) * sizeof(C);
-  if (int rc = allow_smem<coeff_tile_kernel<S, NT, LM>>(TILE_SMEM)) return rc;
+  if (int rc = allow_smem<coeff_tile_kernel<S, NT, LM, SEG>>(TILE_SMEM)) return rc;
   const int64_t blocks = (a.nlines + NT - 1) / NT;
-  coeff_tile_kernel<S, NT, LM><<<static_cast<unsigned>(blocks), TILE_THREADS, smem, st>>>(a);
+  coeff_tile_kernel<S, NT, LM, SEG><<<static_cast<unsigned>(blocks), TILE_THREADS, smem, st>>>(a);
   ppc::count_launch();
   return ppc::cuda_check(cudaGetLastError(), "prefilter launch");
 }
 
-template <class S, int NT>
+template <class S, int NT, bool SEG>
 int launch_tile(const LineArgs& a, cudaStream_t st) {
-  return a.line_major ? launch_tile<S, NT, true>(a, st) : launch_tile<S, NT, false>(a, st);
+  return a.line_major ? launch_tile<S, NT, true, SEG>(a, st) : launch_tile<S, NT, false, SEG>(a, st);
 }
 
 template <class S>
 int launch_tiles(const LineArgs& a, int NT, cudaStream_t st) {
-  if (NT == 128) return launch_tile<S, 128>(a, st);
-  if (NT == 96) return launch_tile<S, 96>(a, st);
-  if (NT == 64) return launch_tile<S, 64>(a, st);
-  return launch_tile<S, 32>(a, st);
+  if constexpr (sizeof(S) < 8) {
+    if (a.nseg > 1) {
+      if (NT == 128) return launch_tile<S, 128, true>(a, st);
+      if (NT == 64) return launch_tile<S, 64, true>(a, st);
+      return launch_tile<S, 32, true>(a, st);
+    }
+  }
+  if (NT == 128) return launch_tile<S, 128, false>(a, st);
+  if (NT == 96) return launch_tile<S, 96, false>(a, st);
+  if (NT == 64) return launch_tile<S, 64, false>(a, st);
+  return launch_tile<S, 32, false>(a, st);
 }
 
 // Whether every line starts on, and consists of, aligned groups of four.  A
