@@ -264,7 +264,7 @@ __device__ __noinline__ void settle(const R& L, int i, int count, bool has, type
 // lines of ordinary volumes only past a stretch of exact zeros) the difference
 // is carried on until all agree: the result is the whole line's.  (The checks
 // cost 2-4 %: 3 x 256^3 cubic 274 -> 280 us for the three axes, 3 x 192^3
-// 125 -> 128 us.)  The warm-ups read what the neighbour is about to overwrite,
+// 125 -> 128 us, one kernel serving whole and cut lines.)  The warm-ups read what the neighbour is about to overwrite,
 // hence the barriers; all threads of the CTA make the call.
 template <class R>
 __device__ void filter_segment(const R& L, int n, const LineArgs& a, int j, bool active) {
@@ -360,8 +360,8 @@ struct alignas(4 * sizeof(S)) Quad {
 // recursions, two dependent passes of n steps, took longer than the
 // transfers: at 64 lines per CTA and four segments of 64 samples (warm-ups of
 // 23) per line of 256, three CTAs per SM, the three axes of 3 x 256^3 floats
-// take 280 us (374 with one thread per line and 96 lines per CTA), 187 us of it
-// memory traffic at the copy rate; 3 x 192^3 128 us (149).  More registers per
+// take 279 us (375 with one thread per line and 96 lines per CTA), 187 us of it
+// memory traffic at the copy rate; 3 x 192^3 127 us (150).  More registers per
 // thread or a fourth CTA per SM gain nothing further.
 //  * filtered axis the fastest (LM): a warp instruction covers 8 groups of
 //    four consecutive samples of 4 lines (128-byte segments), through
@@ -741,10 +741,13 @@ int run_axis(LineArgs& a, cudaStream_t st) {
   {
     const int64_t fit = static_cast<int64_t>(TILE_SMEM / (static_cast<size_t>(a.n) * sizeof(C))) - 4;
     // segments, each longer than a warm-up; with fewer than four their warm-ups
-    // and checks cost what they save (cubic 72^3: 20.3 us in two, 19.0 whole)
+    // and checks cost what they save (cubic 72^3: 20.3 us in two, 19 whole)
     int64_t most = sizeof(C) == 4 ? a.n / (a.warm + 1) : 1;
     if (most < 4) most = 1;
-    const int most_nt = most > 1 ? 64 : 128;
+    // (128 lines in two segments where all are then one wave of two CTAs per SM,
+    // and 64-line tiles a wave of three and a remainder: 192^3, 49 -> 42 us)
+    const bool one_wave = fit >= 128 && a.nlines > 64 * 3 * 148 && a.nlines <= 128 * 2 * 148;
+    const int most_nt = most > 1 && !one_wave ? 64 : 128;
     const int NT = static_cast<int>(std::min<int64_t>(most_nt, fit / 32 * 32));
     if (NT > 0) {
       a.nseg = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(TILE_THREADS / NT, most)));

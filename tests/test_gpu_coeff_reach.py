@@ -58,3 +58,18 @@ def test_reach(order, bound, kind):
             fin = np.isfinite(ref).all(1)
             env = _envelope(ref[fin], -POLE[order], bound == 6)
             assert (np.abs(out[fin] - ref[fin]) <= 1e-5 * env + 1e-38).all()
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 8e-3)])
+@pytest.mark.parametrize("lines", [28416, 28417, 30001, 37888, 37889])
+def test_many_lines(lines, dtype, tol):
+    """Line counts around one wave of 128-line tiles (two segments per line)."""
+    g = torch.Generator(device="cuda").manual_seed(lines)
+    x = torch.randn(lines, 200, device="cuda", generator=g).to(dtype)
+    x[::1000, 61] = float("nan")
+    ref = coeff.spline_coeff(x.double(), 3, 3)
+    for axis in (-1, 0):
+        out = coeff.spline_coeff(x if axis else x.T.contiguous(), 3, 3, dim=axis).double()
+        out = out if axis else out.T
+        assert torch.equal(out.isnan(), ref.isnan())
+        assert float((out - ref).nan_to_num().abs().max() / ref.nan_to_num().abs().max()) < tol
