@@ -101,13 +101,16 @@ def _enums(bound, interpolation):
 _known_enums = functools.lru_cache(maxsize=256)(_enums)
 # entries that are equal for good; others (a tensor hashes by identity and can
 # change its value) are read anew on each call
-_CONSTANT = (str, int, BoundType, InterpolationType)
+_CONSTANT = frozenset((str, int, BoundType, InterpolationType))
 
 
 def _opt(bound, interpolation, extrapolate):
-    bound, interpolation = tuple(make_list(bound)), tuple(make_list(interpolation))
-    constant = all(type(x) in _CONSTANT for x in bound + interpolation)
-    bound, interpolation = (_known_enums if constant else _enums)(bound, interpolation)
+    if type(bound) in _CONSTANT and type(interpolation) in _CONSTANT:
+        bound, interpolation = _known_enums((bound,), (interpolation,))
+    else:
+        bound, interpolation = tuple(make_list(bound)), tuple(make_list(interpolation))
+        constant = all(type(x) in _CONSTANT for x in bound + interpolation)
+        bound, interpolation = (_known_enums if constant else _enums)(bound, interpolation)
     return list(bound), list(interpolation), int(extrapolate)
 
 

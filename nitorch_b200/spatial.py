@@ -35,6 +35,7 @@ Argument errors raise ``RuntimeError`` with the reference's "(): expected
     second axis' order for the third, ``pushpull_common.cpp:591``).
 """
 import ctypes
+import math
 import os
 import threading
 import weakref
@@ -162,6 +163,7 @@ _BRICK = (4, 4, 6)  # PP_BRICK_X, PP_BRICK_Y, PP_BRICK_Z
 
 
 _INT = (1 << 31) - 1
+_DIRECT_DTYPES = (torch.float32, torch.bfloat16)
 _direct_enabled = not os.environ.get("PP_PUSH_LANES", "").startswith("0")
 
 
@@ -189,20 +191,26 @@ def _direct(grid, src_size, interpolation, images):
     466 / 304), and "sorted" is faster for them."""
     if images is None or _deterministic or not _direct_enabled or grid.dtype != torch.float32:
         return False
-    dtype, channels = (images[0].dtype, images[0].shape[1]) if images else (grid.dtype, 1)
-    dim = grid.dim() - 2
+    first = images[0] if images else None
+    if first is not None and first.dtype not in _DIRECT_DTYPES:
+        return False
+    size = grid.shape
+    dim = len(size) - 2
     order = int(interpolation[0])
-    if dtype not in (torch.float32, torch.bfloat16) or any(int(i) != order for i in interpolation[1:dim]):
+    if len(interpolation) > 1 and any(int(i) != order for i in interpolation[1:dim]):
         return False
-    if not (order in (1, 2, 3) if dim == 2 else dim == 3 and (order == 1 or order == 2 and channels == 1)):
+    if dim == 3:
+        if not (order == 1 or order == 2 and (first is None or first.shape[1] == 1)):
+            return False
+    elif dim != 2 or order not in (1, 2, 3):
         return False
-    planes = grid.shape[0] * (grid.shape[1] if dim == 3 else 1)
-    source = 1
-    for n in src_size:
-        source *= int(n)
-    return (planes < (1 << 24) and grid.shape[dim - 1] <= 65535 and grid.numel() // grid.shape[0] < _INT
-            and grid.numel() // dim < _INT and source < _INT and _extent_fits(grid)
-            and all(_extent_fits(t) for t in images))
+    if size[dim - 1] > 65535:
+        return False
+    n = grid.numel()
+    if n >= 1 << 24 and not ((size[0] * size[1] if dim == 3 else size[0]) < (1 << 24) and n // size[0] < _INT
+                             and n // dim < _INT):
+        return False
+    return math.prod(src_size) < _INT and _extent_fits(grid) and all(map(_extent_fits, images))
 
 
 def _brick_least(op, interpolation):
