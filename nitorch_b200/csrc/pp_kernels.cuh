@@ -126,8 +126,22 @@ __device__ __forceinline__ void build_axis(Axis<NT, T, I>& ax, int ORDc, int bnd
   x = fmin(fmax(x, T(-1073741824.0)), T(1073741824.0));
   const I low = support_low<I, T>(ord, x);
   const bool inside = low >= 0 && low + nt - 1 < n;
-  const T f = (x - static_cast<T>(low)) - T(0.5) * static_cast<T>(ord - 1);
-  bspline_stencil<NT, NEED_G, NEED_H, T>(ord, ord == 0 ? T(0) : f, ax.w, ax.g, ax.h);
+  if constexpr (std::is_same<T, float>::value && !NEED_H && (NT == 3 || NT == 4)) {
+    // quadratic and cubic (NT is the order's own): the closed form that the
+    // direct and brick kernels use, from the exact fraction, so that a call's
+    // rounding does not depend on which of them takes it
+    const float r = x - floorf(x);
+    spline_weights<NT - 1, NEED_G>(NT == 4 ? r : r < 0.5f ? r + 0.5f : r - 0.5f, ax.w,
+                                   ax.g);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      if (!NEED_G) ax.g[t] = 0.f;
+      ax.h[t] = 0.f;
+    }
+  } else {
+    const T f = (x - static_cast<T>(low)) - T(0.5) * static_cast<T>(ord - 1);
+    bspline_stencil<NT, NEED_G, NEED_H, T>(ord, ord == 0 ? T(0) : f, ax.w, ax.g, ax.h);
+  }
   ax.mask = 0;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {

@@ -70,3 +70,29 @@ def test_small_volumes_run_per_point(n, order, bricks):
     assert not any(k.startswith("pp_direct_") for k in kernels), kernels
     for a, r in zip(out, ref):
         assert float((a - r).abs().max() / r.abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("order", [2, 3])
+def test_rounding_does_not_depend_on_the_order(order):
+    """RMS error against float64 of the gathers that small volumes leave to the
+    per-point kernel: no larger than the brick kernels' (the same weights; sums
+    in another order: margin 1.1)."""
+    g = torch.Generator(device="cuda").manual_seed(order)
+    image = torch.rand(1, 3, 40, 41, 42, device="cuda", generator=g).requires_grad_()
+    grid = (torch.rand(1, 60, 61, 62, 3, device="cuda", generator=g) * 38 + 1).requires_grad_()
+    target = torch.rand(1, 3, 60, 61, 62, device="cuda", generator=g)
+    b, o = enums(2, order)
+
+    def run(dt):
+        x, p, t = (v.detach().to(dt).requires_grad_() for v in (image, grid, target))
+        return [spatial.grid_pull(x, p, b, o, 1), spatial.grid_grad(x, p, b, o, 1), *spatial.grid_push_backward(x.detach(), t, p, b, o, 1)]
+
+    errors = {}
+    ref = run(torch.float64)
+    for mode in ("natural", "sorted"):
+        spatial.set_sample_order(mode)
+        out = run(torch.float32)
+        assert _lib.last_kernel().startswith("pp_brick_" if mode == "sorted" else ("pp_direct", "pp_kernel", "pp_lanes"))
+        errors[mode] = [float((a.double() - r).pow(2).mean().sqrt()) for a, r in zip(out, ref)]
+    for a, r in zip(errors["natural"], errors["sorted"]):
+        assert a <= 1.1 * r, errors
